@@ -266,8 +266,9 @@ PASTIX_GPU_API int pastix_gpu_phase_log( pastix_gpu_t *ctx, int64_t *count, int6
  *   PGPU_TUNE_TRSM_GEMM       1 (default): tall panels' TRSM as a GEMM against the inverse
  *   PGPU_TUNE_TRSM_GEMM_ROWS  panel height above which it applies (256)
  *   PGPU_TUNE_TC_MIN_MN       smallest M x N update sent to the tensor cores (8192)
- *   PGPU_TUNE_WIDE_PANEL      narrowest diagonal block factorized by the 512-thread
- *                             left-looking kernel (128; 0 disables it)
+ *   PGPU_TUNE_WIDE_PANEL      narrowest diagonal block always factorized one CTA per
+ *                             32-row block row (128; those of 33 columns and more are
+ *                             too where a level has few of them; 0 disables it)
  *   PGPU_TUNE_TC_TMA          1 (default): split operands (3xFP16 / 3xTF32) pre-split once per
  *                             panel and loaded by TMA; 0: 3xTF32 split by producer warps per tile
  *   PGPU_TUNE_TC_PAIR_MIN     TMA kernel: fewest tiles in a launch for pairing 128-row

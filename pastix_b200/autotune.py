@@ -8,8 +8,8 @@ library's CUDA events), by coordinate descent over a small candidate space:
   trsm_gemm_rows   panel height above which the TRSM runs as a GEMM
   tc_min_mn        smallest M x N update sent to the tensor cores
   la_reserved_sms  SMs the lookahead stream leaves to the critical path
-  wide_panel       narrowest diagonal block given to the left-looking
-                   512-thread panel kernel (0: none)
+  wide_panel       narrowest diagonal block always given to the block-row
+                   panel kernel (0: none)
   mixed_gemm       3xFP16 vs 3xTF32 vs one TF32 product (objective "solve": the
                    refinement's extra iterations are part of the cost)
 

@@ -6,7 +6,8 @@
 #include "pgpu_solve.cuh"
 #include "pgpu_panel.cuh"
 #include "pgpu_gemm_tc.cuh"
-#include "pgpu_panel_wide.cuh"
+#include "pgpu_panel_rows.cuh"
+#include "pgpu_panel_small.cuh"
 #include "pgpu_gemm_tma.cuh"
 #include "pgpu_gemm_f64.cuh"
 #include "pgpu_spm.cuh"
@@ -129,11 +130,19 @@ struct pastix_gpu_s {
     int plan_fact = -1;
     std::vector<int> tile_ptr, tctile_ptr, trsm_ptr, lvl_plrows, lvl_porows;
     std::vector<int> stile_n;   // per level and part (next-level targets, others): warp tiles at the part's end
-    // panel launches of a level: k_panel_factor over the narrow cblks and
-    // k_panel_wide over the wide diagonal blocks, jobs {cblk, position in
+    // panel launches of a level: k_panel_factor, jobs {cblk, position in
     // lvl_cblks} (the position indexes the task records)
-    std::vector<int> pn_ptr, pw_ptr, lvl_pmaxw, lvl_wmaxw;
-    DArr<int2> d_pjobs, d_wjobs;
+    std::vector<int> pn_ptr, lvl_pmaxw;
+    DArr<int2> d_pjobs;
+    // diagonal blocks taken one CTA per block row (k_panel_rows): jobs, and per
+    // level the staging slots and shared memory of its widest block; counters
+    // (one per block row of the plan, then one ticket per level), published tiles
+    std::vector<int> pr_ptr, pr_lslots;
+    std::vector<size_t> pr_lsmem;
+    DArr<int4> d_prjobs;
+    DArr<int> d_prog;
+    DArr<unsigned char> d_prscr;
+    int pr_counters = 0;
     std::vector<int> ps_ptr;   // cblks of at most 32 columns: one warp each (k_panel_small)
     DArr<int2> d_sjobs;
     DArr<int4> d_tiles, d_tctiles, d_trsm;
@@ -232,6 +241,7 @@ struct pastix_gpu_s {
     std::vector<int> split_ptr;
     DArr<int4> d_split;
     std::vector<int> inv_ptr, ttile_ptr, tttile_ptr;   // per level: inverse jobs, TRSM FMA / TC tiles
+    std::vector<char> lvl_inv;                          // per level: some cblk holds its diagonal block's inverse
     DArr<int2> d_invjobs;
     DArr<int4> d_ttiles, d_tttiles;
     std::vector<int4> h_tiles, h_tctiles, h_trsm;   // host copies of the plan's launch lists
@@ -544,7 +554,7 @@ extern "C" int pastix_gpu_spm(pastix_gpu_t *ctx, int mtxtype, int flttype, int64
 }
 
 static const int SMEM_LIMIT = 227 * 1024;   // opt-in shared memory per CTA
-static const int WP_SMEM_LIMIT = SMEM_LIMIT - 1024;   // k_panel_wide's dynamic part (it has static arrays)
+static const int WP_SMEM_LIMIT = SMEM_LIMIT - 2048;   // dynamic part of kernels with static arrays
 
 // --------------------------------------------------------------------------
 // Factorization plan for one factorization type.
@@ -665,19 +675,17 @@ static int fact_mode_of(int fact, bool zc) {
 }
 
 
-// Chunk width (bytes per row) of k_panel_wide for width w: the widest of
-// 128 / 64 / 32 bytes whose buffers fit in shared memory, 0 if none does.
-static int wide_kcb(int w, size_t esz, bool lu, bool ldl) {
-    for (int kcb = 128; kcb >= 32; kcb /= 2)
-        if (wp_smem_bytes(w, esz, lu, ldl, kcb) <= (size_t)WP_SMEM_LIMIT) return kcb;
-    return 0;
-}
-// Diagonal blocks at least PGPU_TUNE_WIDE_PANEL columns wide (0: never)
-// are factorized by k_panel_wide, when one CTA covers them (elements of up
-// to 8 bytes).
-static bool wide_panel(const pastix_gpu_t &C, int w, size_t esz, bool lu, bool ldl) {
+// Whether k_panel_rows takes a diagonal block of w columns in a level with
+// `nlvl` blocks it could take: PGPU_TUNE_WIDE_PANEL columns or more always
+// (0: none at all), narrower ones where the level has few of them: the one-CTA
+// form (k_panel_factor) finishes a 64-column panel in about the time its block
+// rows take to hand over one tile each, and leaves the other SMs to the rest
+// of a level of thousands; below four such blocks per SM the chain counts
+// (20^3 FP64, levels of 1-16 blocks: 1.33 -> 0.52 ms of panels).
+const int PR_FEW = 592;
+static bool rows_panel(const pastix_gpu_t &C, int w, size_t esz, bool lu, int nlvl) {
     const int64_t wmin = C.tune[PGPU_TUNE_WIDE_PANEL];
-    return wmin > 0 && w >= wmin && esz <= 8 && wp_tiles_fit(w, lu) && wide_kcb(w, esz, lu, ldl) > 0;
+    return wmin > 0 && !C.record && w > PB && (w >= wmin || nlvl <= PR_FEW) && pr_slots(w, esz, lu, WP_SMEM_LIMIT) > 0;
 }
 
 // Forget the captured factorization graph (its nodes name the plan's and the
@@ -900,6 +908,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     std::vector<int4> ttiles, tttiles;
     int64_t inv_elems = 0, scr_max = 0;
     C.inv_ptr.assign(C.nlevels + 1, 0);
+    C.lvl_inv.assign(C.nlevels, 0);
     C.ttile_ptr.assign(C.nlevels + 1, 0);
     C.tttile_ptr.assign(C.nlevels + 1, 0);
     C.invoff.assign(C.cblknbr, -1);
@@ -915,10 +924,16 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     C.lvl_plrows.assign(C.nlevels, 0);
     C.lvl_porows.assign(C.nlevels, 0);
     C.lvl_pmaxw.assign(C.nlevels, 0);
-    C.lvl_wmaxw.assign(C.nlevels, 0);
     C.pn_ptr.assign(C.nlevels + 1, 0);
-    C.pw_ptr.assign(C.nlevels + 1, 0);
-    std::vector<int2> pjobs, wjobs, sjobs;
+    std::vector<int2> pjobs, sjobs;
+    std::vector<int4> prjobs;
+    C.pr_ptr.assign(C.nlevels + 1, 0);
+    C.pr_lslots.assign(C.nlevels, 0);
+    C.pr_lsmem.assign(C.nlevels, 0);
+    C.pr_counters = 0;
+    int64_t prscr_max = 0;
+    // (the 3xTF32 mode's inverse writes its hi / lo planes itself: k_tri_inverse)
+    const bool rows_inv = !(fp32 && !zc && mixed_gemm_mode(C) == MG_3XTF32);
     C.ps_ptr.assign(C.nlevels + 1, 0);
     C.tile_crit.assign(C.nlevels, 0);
     C.tctile_crit.assign(C.nlevels, 0);
@@ -929,6 +944,8 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     C.stile_n.assign(2 * C.nlevels, 0);
     for (int l = 0; l < C.nlevels; l++) {
         int64_t scr_lvl = 0;
+        int prscr = 0, pr_wmax = 0, nlvl = 0;
+        for (int q = C.lvl_ptr[l]; q < C.lvl_ptr[l + 1]; q++) nlvl += C.width[C.lvl_cblks[q]] > PB;
         for (int k = 0; k < 2; k++) {
             lt[k].clear();
             ltc[k].clear();
@@ -937,9 +954,24 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             const int c = C.lvl_cblks[q];
             const int w = C.width[c], h = C.height[c];
             const int rows = (h <= fuse) ? h : w;
-            if (rows == w && wide_panel(C, w, esz, lu, ldl)) {
-                wjobs.push_back(make_int2(c, q));
-                C.lvl_wmaxw[l] = std::max(C.lvl_wmaxw[l], w);
+            const bool by_rows = rows_panel(C, w, esz, lu, nlvl);
+            const int nt = cdiv(w, PB), pr_cnt = C.pr_counters, pr_tile = prscr;
+            // the jobs that invert the diagonal block (after the panel's own)
+            auto inverse_jobs = [&](int sides) {
+                C.lvl_inv[l] = 1;
+                for (int kind = 0; kind < sides; kind++)
+                    for (int jb = 0; jb < nt; jb++) {
+                        if (by_rows && rows_inv)
+                            prjobs.push_back(make_int4(c, jb | ((PR_INV + kind) << 16), pr_cnt, pr_tile));
+                        else
+                            invjobs.push_back(make_int2(c, jb * PB + (kind << 20)));
+                    }
+            };
+            if (by_rows) {
+                for (int i = 0; i < nt + cdiv(rows - w, PB); i++) prjobs.push_back(make_int4(c, i, pr_cnt, pr_tile));
+                C.pr_counters += nt;
+                prscr += nt;
+                pr_wmax = std::max(pr_wmax, w);
             } else if (w <= PB && esz <= 8 && !C.record) {
                 sjobs.push_back(make_int2(c, q));   // one 32-column tile: one warp
             } else {
@@ -959,8 +991,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 const int sides = lu ? 2 : 1;
                 C.invoff[c] = inv_elems;
                 inv_elems += sides * inv_span(w, C.ld[c]);
-                for (int kind = 0; kind < sides; kind++)
-                    for (int jb = 0; jb < w; jb += PB) invjobs.push_back(make_int2(c, jb + (kind << 20)));
+                inverse_jobs(sides);
                 C.scroff[c] = scr_lvl;
                 scr_lvl += sides * inv_span(h - w, C.ld[c]);
                 for (int side = 0; side < sides; side++) {
@@ -979,8 +1010,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 const int sides = lu ? 2 : 1;
                 C.invoff[c] = inv_elems;
                 inv_elems += sides * inv_span(w, C.ld[c]);
-                for (int kind = 0; kind < sides; kind++)
-                    for (int jb = 0; jb < w; jb += PB) invjobs.push_back(make_int2(c, jb + (kind << 20)));
+                inverse_jobs(sides);
             }
             const int b1 = C.fblok[c + 1];
             for (int b = C.fblok[c] + 1; b < b1; b++) {
@@ -1037,7 +1067,12 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
         C.trsm_ptr[l + 1] = (int)trsm.size();
         C.pn_ptr[l + 1] = (int)pjobs.size();
         C.ps_ptr[l + 1] = (int)sjobs.size();
-        C.pw_ptr[l + 1] = (int)wjobs.size();
+        C.pr_ptr[l + 1] = (int)prjobs.size();
+        if (prscr) {
+            C.pr_lslots[l] = pr_slots(pr_wmax, esz, lu, WP_SMEM_LIMIT);
+            C.pr_lsmem[l] = pr_smem_bytes(pr_wmax, esz, lu, C.pr_lslots[l]);
+            prscr_max = std::max<int64_t>(prscr_max, prscr);
+        }
         C.inv_ptr[l + 1] = (int)invjobs.size();
         C.ttile_ptr[l + 1] = (int)ttiles.size();
         C.tttile_ptr[l + 1] = (int)tttiles.size();
@@ -1327,7 +1362,12 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     }
     PGPU_CHECK(C.d_pjobs.upload(pjobs, s));
     PGPU_CHECK(C.d_sjobs.upload(sjobs, s));
-    PGPU_CHECK(C.d_wjobs.upload(wjobs, s));
+    PGPU_CHECK(C.d_prjobs.upload(prjobs, s));
+    if (C.d_prog.n < (size_t)(C.pr_counters + C.nlevels)) PGPU_CHECK(C.d_prog.alloc(C.pr_counters + C.nlevels));
+    if (C.d_prscr.n < (size_t)prscr_max * pr_scr_tile(lu) * esz) {
+        C.d_prscr.release();
+        PGPU_CHECK(C.d_prscr.alloc((size_t)prscr_max * pr_scr_tile(lu) * esz));
+    }
     {
         int rc = build_flow_plan(C, esz, lu);
         if (rc) return rc;
@@ -1391,7 +1431,7 @@ enum { PH_DIAG = 0, PH_TRSM = 1, PH_GEMM = 2, PH_TC = 3, PH_END = 4 };
 template <typename T>
 using PanelKernel = void (*)(Meta, const int2 *, T *, T *, const double *, int, int, int, Status *, int64_t *);
 template <typename T>
-using WideKernel = void (*)(Meta, const int2 *, T *, const double *, int, Status *, int64_t *);
+using RowsKernel = void (*)(Meta, const int4 *, int *, int *, T *, T *, T *, T *, const double *, int, int, Status *);
 
 template <typename T>
 using SmallPanelKernel = void (*)(Meta, const int2 *, int, T *, T *, const double *, int, Status *);
@@ -1412,18 +1452,14 @@ static SmallPanelKernel<T> panel_small_kernel(int fmode) {
 }
 
 template <typename T>
-static WideKernel<T> wide_kernel(int fmode) {
-    if constexpr (sizeof(T) > 8) {
+static RowsKernel<T> rows_kernel(int fmode) {
+    switch (fmode) {
+    case FM_GETRF: return k_panel_rows<T, FM_GETRF>;
+    case FM_SYTRF: return k_panel_rows<T, FM_SYTRF>;
+    case FM_HETRF:
+        if constexpr (is_cplx<T>::value) return k_panel_rows<T, FM_HETRF>;
         return nullptr;
-    } else {
-        switch (fmode) {
-        case FM_GETRF: return k_panel_wide<T, FM_GETRF>;
-        case FM_SYTRF: return k_panel_wide<T, FM_SYTRF>;
-        case FM_HETRF:
-            if constexpr (is_cplx<T>::value) return k_panel_wide<T, FM_HETRF>;
-            return nullptr;
-        default: return k_panel_wide<T, FM_POTRF>;
-        }
+    default: return k_panel_rows<T, FM_POTRF>;
     }
 }
 
@@ -1459,9 +1495,10 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
     if constexpr (sizeof(T) <= 8)
         PGPU_CHECK(cudaFuncSetAttribute(k_gemm_scatter_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         gs_smem_bytes<T>()));
-    WideKernel<T> kwide = wide_kernel<T>(fmode);
-    if (kwide)
-        PGPU_CHECK(cudaFuncSetAttribute(kwide, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM_LIMIT));
+    RowsKernel<T> krows = rows_kernel<T>(fmode);
+    if (!krows) return PASTIX_GPU_ERR_NOTIMPLEMENTED;
+    PGPU_CHECK(cudaFuncSetAttribute(krows, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM_LIMIT));
+    PGPU_CHECK(cudaMemsetAsync(C.d_prog.p, 0, (size_t)(C.pr_counters + C.nlevels) * sizeof(int), s));
     // the Hermitian forms conjugate the L coefficients in the row solves
     constexpr bool CPX = is_cplx<T>::value;
     auto ktrsm = (CPX && fm_conj(fmode)) ? k_trsm_rows<T, TRSM_TR, CPX> : k_trsm_rows<T, TRSM_TR, false>;
@@ -1611,29 +1648,13 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
         }
         const int mw = C.lvl_maxw[l];
         PGPU_CHECK(tm.mark(PH_DIAG));
-        const int npw = C.pw_ptr[l + 1] - C.pw_ptr[l], npn = C.pn_ptr[l + 1] - C.pn_ptr[l];
-        if (npw) {
-            // wide diagonal blocks first: they are the level's longest panels
-            const int wmw = C.lvl_wmaxw[l];
-            const int kcb = wide_kcb(wmw, sizeof(T), lu, fm_ldl(fmode));
-            if (!kwide || kcb == 0) return PASTIX_GPU_ERR_NOTIMPLEMENTED;
-            bool done = false;
-            if constexpr (std::is_same<T, float>::value) {
-                // single-precision LL^t / LDL^t: the lookahead form when its two block columns fit
-                static const bool la_off = getenv("PASTIX_GPU_WIDE_LA") && std::strcmp(getenv("PASTIX_GPU_WIDE_LA"), "0") == 0;
-                const size_t lsm = wpla_smem_bytes(wmw, fm_ldl(fmode));
-                if (!la_off && (fmode == FM_POTRF || fmode == FM_SYTRF) && lsm <= (size_t)WP_SMEM_LIMIT &&
-                    wp_row_groups(wmw) * 8 <= 2 * (WP_THREADS - 32)) {
-                    auto kla = fmode == FM_POTRF ? k_panel_wide_la<FM_POTRF> : k_panel_wide_la<FM_SYTRF>;
-                    PGPU_CHECK(cudaFuncSetAttribute(kla, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM_LIMIT));
-                    kla<<<npw, WP_THREADS, lsm, s>>>(C.meta, C.d_wjobs.p + C.pw_ptr[l], coefL, critp, C.d_status.p,
-                                                     prof[0]);
-                    done = true;
-                }
-            }
-            if (!done)
-                kwide<<<npw, WP_THREADS, wp_smem_bytes(wmw, sizeof(T), lu, fm_ldl(fmode), kcb), s>>>(
-                    C.meta, C.d_wjobs.p + C.pw_ptr[l], coefL, critp, kcb / (int)sizeof(T), C.d_status.p, prof[0]);
+        const int npr = C.pr_ptr[l + 1] - C.pr_ptr[l], npn = C.pn_ptr[l + 1] - C.pn_ptr[l];
+        if (npr) {
+            // the block rows first: they are the level's longest panels
+            krows<<<npr, PR_THREADS, C.pr_lsmem[l], s>>>(
+                C.meta, C.d_prjobs.p + C.pr_ptr[l], C.d_prog.p + C.pr_counters + l, C.d_prog.p,
+                reinterpret_cast<T *>(C.d_prscr.p), coefL, coefU, reinterpret_cast<T *>(C.d_inv.p), critp, fuse,
+                C.pr_lslots[l], C.d_status.p);
             nl++;
         }
         if constexpr (sizeof(T) <= 8) {
@@ -1677,12 +1698,14 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
             const int bulk_lb = bsm <= (size_t)WP_SMEM_LIMIT ? slb : 0;
             if (bulk_lb) ism = std::max(ism, bsm);
             PGPU_CHECK(tm.mark(PH_TRSM));
-            k_tri_inverse<T><<<nij, 256, ism, s>>>(C.meta, C.d_invjobs.p + C.inv_ptr[l], coefL, inv,
-                                                   fm_ldl(fmode) ? 1 : 0, (CPX && fm_conj(fmode)) ? 1 : 0,
-                                                   fm_ldl(fmode) ? 1 : 0, lu ? 1 : 0, kch,
-                                                   (C.tma && !C.h16) ? hilo_of<T>(C.d_ihilo.p) : nullptr,
-                                                   C.ihilo_plane, bulk_lb, C.d_status.p);
-            nl++;
+            if (nij) {
+                k_tri_inverse<T><<<nij, 256, ism, s>>>(C.meta, C.d_invjobs.p + C.inv_ptr[l], coefL, inv,
+                                                       fm_ldl(fmode) ? 1 : 0, (CPX && fm_conj(fmode)) ? 1 : 0,
+                                                       fm_ldl(fmode) ? 1 : 0, lu ? 1 : 0, kch,
+                                                       (C.tma && !C.h16) ? hilo_of<T>(C.d_ihilo.p) : nullptr,
+                                                       C.ihilo_plane, bulk_lb, C.d_status.p);
+                nl++;
+            }
             split_level(l);
             const int ntt = C.ttile_ptr[l + 1] - C.ttile_ptr[l];
             if (ntt) {
@@ -2044,6 +2067,7 @@ static int flow_launch(pastix_gpu_t &C, bool fwd, int run, const T *coefL, const
     a.Y = reinterpret_cast<T *>(C.d_flowY.p);
     a.Z = reinterpret_cast<T *>(C.d_flowZ.p);
     a.ldb = ldb;
+    a.nv = nv;
     a.ldl = ldl ? 1 : 0;
     a.cjp = cjp;
     a.vec_elems = vec_elems;
@@ -2159,7 +2183,7 @@ static int solve_permuted(pastix_gpu_t &C, T *W, int nrhs, int *launches, int st
         const size_t fixed = ((size_t)mw * nrhs + 32 * 33) * es;
         size_t dsm;
         *ipch = 0;
-        if (inv && C.inv_ptr[l + 1] > C.inv_ptr[l]) {
+        if (inv && C.lvl_inv[l]) {
             // rows of the inverse are staged padded to 16 bytes
             const size_t rowb = (size_t)round_up(mw, 16 / (int64_t)es) * es;
             const size_t fixed_i = ((size_t)2 * mw * nrhs + 16) * es;   // + alignment of the staged rows
@@ -2210,10 +2234,10 @@ static int solve_permuted(pastix_gpu_t &C, T *W, int nrhs, int *launches, int st
         int pch = 0;
         int ipch = 0;
         const size_t dsm = diag_smem(l, mw, &pch, &ipch);
-        if (pch < std::min(32, mw) || (inv && C.inv_ptr[l + 1] > C.inv_ptr[l] && ipch < 1))
+        if (pch < std::min(32, mw) || (inv && C.lvl_inv[l] && ipch < 1))
             return PASTIX_GPU_ERR_NOTIMPLEMENTED;
         PGPU_CHECK(mark(0));
-        const int dthreads = (inv && C.inv_ptr[l + 1] > C.inv_ptr[l]) ? 1024 : 256;
+        const int dthreads = (inv && C.lvl_inv[l]) ? 1024 : 256;
         k_fwd_diag<T><<<ncb, dthreads, dsm, s>>>(
             C.meta, C.d_lvl_cblks.p + C.lvl_ptr[l], coefL, W, ldb, nrhs, (lu || ldl) ? 1 : 0, pch, inv,
             ldl ? 1 : 0, cjp, ipch);
@@ -2291,7 +2315,7 @@ static int solve_permuted(pastix_gpu_t &C, T *W, int nrhs, int *launches, int st
         int ipch = 0;
         const size_t dsm = diag_smem(l, mw, &pch, &ipch);
         PGPU_CHECK(mark(4));
-        const int dthreads = (inv && C.inv_ptr[l + 1] > C.inv_ptr[l]) ? 1024 : 256;
+        const int dthreads = (inv && C.lvl_inv[l]) ? 1024 : 256;
         k_bwd_diag<T><<<ncb, dthreads, dsm, s>>>(C.meta, C.d_lvl_cblks.p + C.lvl_ptr[l], coefL, W, ldb, nrhs,
                                             lu ? 1 : 0, ldl ? 1 : 0, lu ? 0 : cjp, pch, inv, ldl ? 1 : 0, ipch);
         nl++;
