@@ -277,8 +277,9 @@ PASTIX_GPU_API int pastix_gpu_phase_log( pastix_gpu_t *ctx, int64_t *count, int6
  *                             for a 128 x 64 tile on the FP64 tensor cores (DMMA); 0: FMA tiles
  *   PGPU_TUNE_SOLVE_FLOW      1 (default): runs of solve levels whose cblks all hold a
  *                             diagonal-block inverse go through one dataflow launch per
- *                             direction (per-cblk counters instead of per-level launches;
- *                             1, 2 or 4 right-hand sides, complex128: 1 or 2); 0: per-level launches
+ *                             direction (per-cblk counters instead of per-level launches; any
+ *                             number of right-hand sides, 8 at a time in single precision,
+ *                             4 in FP64 and complex64, 2 in complex128); 0: per-level launches
  *   PGPU_TUNE_GRAPH           -1 (default): the factorization captured as a CUDA graph and
  *                             replayed when the factor holds at most 2^24 coefficients
  *                             (launch-bound sizes); 1 always; 0 never

@@ -221,7 +221,7 @@ struct pastix_gpu_s {
     // inverse (k_solve_flow): runs {first level, end level}, per run the task
     // ranges (forward, backward), the per-cblk counters (5 x cblknbr) and their
     // per-launch increments (4 x cblknbr), epochs and ticket bases, the Y and Z
-    // blocks (n x FLOW_MAXRHS each), the largest width of a run's cblk
+    // blocks (n x flow_maxrhs each), the largest width of a run's cblk
     std::vector<int2> flow_runs;
     std::vector<int> flow_tptr[2];    // per run: first task
     DArr<int> d_flow_off[2];          // per run: 2 x (G + 1) offsets of the CTAs' tasks in the two lists
@@ -711,7 +711,7 @@ static int flow_reset(pastix_gpu_t &C) {
 // Runs of consecutive levels the dataflow solve takes (k_solve_flow): levels
 // that are not solved one warp per cblk and whose cblks all hold the inverse
 // of their diagonal block (and narrow enough for one stage's vector part of
-// FLOW_MAXRHS right-hand sides, complex128: 2).  Tasks of at most
+// flow_maxrhs right-hand sides).  Tasks of at most
 // FLOW_MAXROWS rows (fewer where a row is long: one staging buffer), in two
 // lists per direction -- critical: the diagonal tasks and the updates of a
 // cblk of the next level; the others -- each sorted by one key that is a
@@ -728,7 +728,7 @@ static int flow_reset(pastix_gpu_t &C) {
 // key of the task that needs it (backward G: 2 d(c)) -- by which the fetch
 // warp chooses between the heads of its two lists.  List task i goes to CTA
 // i mod G (G: one CTA per SM); the lists are stored CTA by CTA.  Y and Z for
-// up to FLOW_MAXRHS right-hand sides are allocated here, with the plan (the
+// up to flow_maxrhs right-hand sides are allocated here, with the plan (the
 // allocation-free solve allocates nothing).
 static int build_flow_plan(pastix_gpu_t &C, size_t esz, bool lu) {
     C.flow_runs.clear();
@@ -740,7 +740,7 @@ static int build_flow_plan(pastix_gpu_t &C, size_t esz, bool lu) {
         bool all = !(C.lvl_maxw[l] <= 32 && C.lvl_maxh[l] <= SOLVE_SMALL_MAXH) && C.lvl_ptr[l + 1] > C.lvl_ptr[l];
         for (int q = C.lvl_ptr[l]; q < C.lvl_ptr[l + 1] && all; q++) {
             const int c = C.lvl_cblks[q];
-            const size_t vmax = (size_t)std::max(C.width[c], FLOW_MAXROWS) * (esz <= 8 ? FLOW_MAXRHS : 2) * esz;
+            const size_t vmax = (size_t)std::max(C.width[c], FLOW_MAXROWS) * flow_maxrhs(esz) * esz;
             all = C.invoff[c] >= 0 && vmax + 16 <= (size_t)FLOW_VEC_BYTES && (size_t)C.ld[c] * esz <= (size_t)FLOW_STAGE;
         }
         ok[l] = all;
@@ -871,7 +871,7 @@ static int build_flow_plan(pastix_gpu_t &C, size_t esz, bool lu) {
         C.d_flow_cnt.release();
         PGPU_CHECK(C.d_flow_cnt.alloc(5 * (size_t)nc));
     }
-    const size_t vbytes = (size_t)C.n * FLOW_MAXRHS * esz;
+    const size_t vbytes = (size_t)C.n * flow_maxrhs(esz) * esz;
     if (C.d_flowY.n < vbytes) {
         C.d_flowY.release();
         PGPU_CHECK(C.d_flowY.alloc(vbytes));
@@ -2032,11 +2032,11 @@ extern "C" int pastix_gpu_numfact(pastix_gpu_t *ctx, const void *values) {
 // One launch of the dataflow solve over run `run`, forward or backward: a
 // cooperative launch (every CTA resident), one CTA per SM.
 template <typename T, int NR>
-static int flow_launch(pastix_gpu_t &C, bool fwd, int run, const T *coefL, const T *inv, T *W, int ldb, bool ldl,
-                       int cjp) {
+static int flow_launch(pastix_gpu_t &C, int nv, bool fwd, int run, const T *coefL, const T *inv, T *W, int ldb,
+                       bool ldl, int cjp) {
     const int dir = fwd ? 0 : 1;
     auto kern = fwd ? k_solve_flow<T, NR, true> : k_solve_flow<T, NR, false>;
-    const int vec_elems = (int)align16_elems<T>((size_t)std::max(C.flow_maxw, FLOW_MAXROWS) * NR);
+    const int vec_elems = (int)align16_elems<T>((size_t)std::max(C.flow_maxw, FLOW_MAXROWS)) * NR;
     const size_t smem = (size_t)FLOW_S * FLOW_STAGE + (size_t)FLOW_S * vec_elems * sizeof(T);
     if ((size_t)vec_elems * sizeof(T) > (size_t)FLOW_VEC_BYTES) return PASTIX_GPU_ERR_INTERNAL;
     static size_t attr[2] = {0, 0};   // dynamic shared memory the kernel is set up for
@@ -2118,17 +2118,34 @@ static int flow_launch(pastix_gpu_t &C, bool fwd, int run, const T *coefL, const
     return PASTIX_GPU_SUCCESS;
 }
 
+// One run over all nrhs right-hand sides, flow_maxrhs at a time (each pass
+// reads the factor once, so as many as fit; the last pass takes the smallest
+// kernel that holds what is left, its surplus columns zero).
 template <typename T>
 static int flow_launch_nr(pastix_gpu_t &C, int nrhs, bool fwd, int run, const T *coefL, const T *inv, T *W,
-                          int ldb, bool ldl, int cjp) {
-    switch (nrhs) {
-    case 1: return flow_launch<T, 1>(C, fwd, run, coefL, inv, W, ldb, ldl, cjp);
-    case 2: return flow_launch<T, 2>(C, fwd, run, coefL, inv, W, ldb, ldl, cjp);
-    case 4:
-        if constexpr (sizeof(T) <= 8) return flow_launch<T, 4>(C, fwd, run, coefL, inv, W, ldb, ldl, cjp);
-        return PASTIX_GPU_ERR_INTERNAL;
-    default: return PASTIX_GPU_ERR_INTERNAL;
+                          int ldb, bool ldl, int cjp, int *launches) {
+    constexpr int MAXR = flow_maxrhs(sizeof(T));
+    for (int r0 = 0; r0 < nrhs; r0 += MAXR) {
+        const int nv = std::min(MAXR, nrhs - r0);
+        T *Wr = W + (int64_t)r0 * ldb;
+        int rc;
+        if (nv == 1) {
+            rc = flow_launch<T, 1>(C, nv, fwd, run, coefL, inv, Wr, ldb, ldl, cjp);
+        } else if (nv == 2) {
+            rc = flow_launch<T, 2>(C, nv, fwd, run, coefL, inv, Wr, ldb, ldl, cjp);
+        } else if constexpr (MAXR >= 4) {
+            if constexpr (MAXR >= 8)
+                rc = nv > 4 ? flow_launch<T, 8>(C, nv, fwd, run, coefL, inv, Wr, ldb, ldl, cjp)
+                            : flow_launch<T, 4>(C, nv, fwd, run, coefL, inv, Wr, ldb, ldl, cjp);
+            else
+                rc = flow_launch<T, 4>(C, nv, fwd, run, coefL, inv, Wr, ldb, ldl, cjp);
+        } else {
+            rc = PASTIX_GPU_ERR_INTERNAL;
+        }
+        if (rc) return rc;
+        ++*launches;
     }
+    return PASTIX_GPU_SUCCESS;
 }
 
 // A wait of the dataflow solve that gave up (FlowState::err): the solve's
@@ -2198,8 +2215,7 @@ static int solve_permuted(pastix_gpu_t &C, T *W, int nrhs, int *launches, int st
     // levels of narrow, short cblks: one warp per cblk, diagonal and off-diagonal parts in one launch
     auto small_level = [&](int l) { return C.lvl_maxw[l] <= 32 && C.lvl_maxh[l] <= SOLVE_SMALL_MAXH; };
     // runs of levels with diagonal-block inverses: one dataflow launch each way
-    const bool flow = inv && C.tune[PGPU_TUNE_SOLVE_FLOW] != 0 &&
-                      (nrhs == 1 || nrhs == 2 || (nrhs == 4 && sizeof(T) <= 8)) && nrhs <= FLOW_MAXRHS;
+    const bool flow = inv && C.tune[PGPU_TUNE_SOLVE_FLOW] != 0;
     auto flow_run_at = [&](int l, bool first) {
         if (flow)
             for (size_t r = 0; r < C.flow_runs.size(); r++)
@@ -2213,9 +2229,8 @@ static int solve_permuted(pastix_gpu_t &C, T *W, int nrhs, int *launches, int st
         const int run = flow_run_at(l, true);
         if (run >= 0) {
             PGPU_CHECK(mark(0));
-            int rc = flow_launch_nr<T>(C, nrhs, true, run, coefL, inv, W, ldb, ldl, cjp);
+            int rc = flow_launch_nr<T>(C, nrhs, true, run, coefL, inv, W, ldb, ldl, cjp, &nl);
             if (rc) return rc;
-            nl++;
             l = C.flow_runs[run].y - 1;
             continue;
         }
@@ -2273,9 +2288,8 @@ static int solve_permuted(pastix_gpu_t &C, T *W, int nrhs, int *launches, int st
         const int run = flow_run_at(l, false);
         if (run >= 0) {
             PGPU_CHECK(mark(4));
-            int rc = flow_launch_nr<T>(C, nrhs, false, run, coefL, inv, W, ldb, ldl, lu ? 0 : cjp);
+            int rc = flow_launch_nr<T>(C, nrhs, false, run, coefL, inv, W, ldb, ldl, lu ? 0 : cjp, &nl);
             if (rc) return rc;
-            nl++;
             l = C.flow_runs[run].x;
             continue;
         }

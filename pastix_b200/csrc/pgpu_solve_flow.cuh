@@ -59,7 +59,9 @@ constexpr int FLOW_S = 4;                 // pipeline stages per CTA
 constexpr int FLOW_STAGE = 40 * 1024;     // bytes of one stage's factor rows
 constexpr int FLOW_VEC_BYTES = 16 * 1024;   // bytes of one stage's vector part (at most)
 constexpr int FLOW_MAXROWS = 32;          // rows of the factor per task
-constexpr int FLOW_MAXRHS = 4;            // right-hand sides of one pass (1, 2 or 4; complex128: 1 or 2)
+// right-hand sides of one pass, at most: 32 bytes of them per vector row (8 in single precision, 2 in
+// complex128), which keeps the vector parts of four stages beside the staged rows in shared memory
+__host__ __device__ constexpr int flow_maxrhs(size_t esz) { return 32 / (int)esz; }
 constexpr int FLOW_CWARPS = 8;            // compute warps
 constexpr int FLOW_VWARPS = 4;            // vector warps (stage uses k with k mod 4 = the warp's index)
 constexpr int FLOW_SWARPS = 4;            // signal warps (likewise)
@@ -159,8 +161,9 @@ struct FlowArgs {
     FlowCounters k;
     const T *coef;    // coefficient array (L, then U^t for LU): O / G rows, LDL diagonals
     const T *inv;     // diagonal-block inverses: D / E rows
-    T *B, *Y, *Z;     // right-hand sides (ld ldb), forward y, backward partial sums
+    T *B, *Y, *Z;     // right-hand sides, forward y, backward partial sums (all ld ldb)
     int ldb;
+    int nv;           // right-hand sides of this pass (at most the kernel's NR; the others read as zero)
     int ldl, cjp;     // LDL scaling; conj (forward: inverse and d; backward: the gathered panel)
     int vec_elems;    // elements of one stage's vector part
     unsigned long long *stamps;   // diagnostics (may be null): per task, global timer at compute start and at
@@ -196,6 +199,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_solve_flow(FlowArgs<T> a) {
         return (q.hdr & 7) == FLOW_D ? a.k.go + q.c : a.k.bx + q.f;
     };
     auto data = [&](int s) { return flow_smem + (size_t)s * FLOW_STAGE; };
+    const int vpitch = a.vec_elems / NR;   // forward: one right-hand side's vector (whole 16-byte vectors)
     auto vec_of = [&](int s) {
         return reinterpret_cast<T *>(flow_smem + (size_t)FLOW_S * FLOW_STAGE) + (size_t)s * a.vec_elems;
     };
@@ -367,19 +371,24 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_solve_flow(FlowArgs<T> a) {
             const int kind = q.hdr & 7, nr = (q.hdr >> 4) & 63;
             vbase = vec_of(s);
             const T *Bf = a.B + q.fc;
-            if (FWD && kind == FLOW_D) {   // b_c, columns 0 .. r0 + nr - 1
-                gather((q.r0 + nr) * NR, [&](int e) { return ldcg_v(Bf + (int64_t)(e % NR) * a.ldb + e / NR); });
-            } else if (FWD) {              // y_c, and the rows the task updates
+            if (FWD && kind == FLOW_D) {   // b_c, columns 0 .. r0 + nr - 1, one right-hand side after the other
+                for (int r = 0; r < NR; r++, vbase += vpitch)
+                    gather(q.r0 + nr, [&](int e) { return r < a.nv ? ldcg_v(Bf + (int64_t)r * a.ldb + e) : T(0); });
+            } else if (FWD) {              // y_c alike, and the rows the task updates
                 const T *Yf = a.Y + q.fc;
                 if (lane < nr) rowsm[s][lane] = __ldg(a.m.rowidx + q.aux + lane);
-                gather(q.w * NR, [&](int e) { return ldcg_v(Yf + (int64_t)(e % NR) * a.ldb + e / NR); });
-            } else if (kind == FLOW_O) {   // x at the task's rows
+                for (int r = 0; r < NR; r++, vbase += vpitch)
+                    gather(q.w, [&](int e) { return r < a.nv ? ldcg_v(Yf + (int64_t)r * a.ldb + e) : T(0); });
+            } else if (kind == FLOW_O) {   // x at the task's rows, the right-hand sides of a row together
                 if (lane < nr) rowsm[s][lane] = __ldg(a.m.rowidx + q.aux + lane);
                 __syncwarp();
                 const int *rw = rowsm[s];
-                gather(nr * NR, [&](int e) { return ldcg_v(a.B + (int64_t)(e % NR) * a.ldb + rw[e / NR]); });
+                gather(nr * NR, [&](int e) {
+                    return e % NR < a.nv ? ldcg_v(a.B + (int64_t)(e % NR) * a.ldb + rw[e / NR]) : T(0);
+                });
             } else {                       // v' = d t (LDL) or t, rows r0 ..
                 gather(nr * NR, [&](int e) {
+                    if (e % NR >= a.nv) return T(0);
                     const int n = q.r0 + e / NR;
                     T x = ldcg_v(Bf + (int64_t)(e % NR) * a.ldb + n);
                     if (a.ldl) x = x * a.coef[q.aux + (int64_t)n * q.ld + n];
@@ -410,33 +419,17 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_solve_flow(FlowArgs<T> a) {
             if (FWD) {
                 // D  y_n = s op(Binv[n][k]) b_k, k <= n;  O  b[row_i] -= P[i][k] y_k.  Warp w takes rows
                 // w, w + 8, .. (RW of them) together: lanes across k in 16-byte vectors, each vector of v
-                // loaded once for all RW rows, every load of a pass independent of the others
-                constexpr int VEC = 16 / sizeof(T), RW = FLOW_MAXROWS / FLOW_CWARPS;
+                // loaded once for all RW rows, every load of a pass independent of the others; each
+                // right-hand side's v is contiguous, so its loads are conflict-free for any NR
+                constexpr int VEC = 16 / sizeof(T), RW = FLOW_MAXROWS / FLOW_CWARPS, NA = RW * NR;
                 const bool dk = kind == FLOW_D;
                 const int ilast = min(nr - 1, warp + FLOW_CWARPS * (RW - 1));
                 const int kend = dk ? r0 + ilast + 1 : w;   // columns any of the warp's rows uses
-                T acc[RW][NR];
+                T acc[NA];   // [row u][right-hand side r]
 #pragma unroll
-                for (int u = 0; u < RW; u++)
-#pragma unroll
-                    for (int r = 0; r < NR; r++) acc[u][r] = T(0);
+                for (int u = 0; u < NA; u++) acc[u] = T(0);
                 if (warp < nr) {
                     for (int k0 = lane * VEC; k0 < kend; k0 += 32 * VEC) {
-                        T vv[VEC][NR];
-                        if (NR == 1 && k0 + VEC <= kend) {
-                            T t4[VEC];
-                            const uint4 u4 = lds_u4(sv + (uint32_t)k0 * sizeof(T));   // (16-byte aligned)
-                            memcpy(t4, &u4, 16);
-#pragma unroll
-                            for (int q = 0; q < VEC; q++) vv[q][0] = t4[q];
-                        } else {
-#pragma unroll
-                            for (int q = 0; q < VEC; q++)
-#pragma unroll
-                                for (int r = 0; r < NR; r++)
-                                    vv[q][r] = k0 + q < kend ? lds_t<T>(sv + (uint32_t)((k0 + q) * NR + r) * sizeof(T))
-                                                         : T(0);
-                        }
                         T e[RW][VEC];
 #pragma unroll
                         for (int u = 0; u < RW; u++) {
@@ -445,45 +438,57 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_solve_flow(FlowArgs<T> a) {
                             memcpy(e[u], &u4, 16);
                         }
 #pragma unroll
-                        for (int u = 0; u < RW; u++) {
-                            const int klim = dk ? r0 + warp + FLOW_CWARPS * u + 1 : w;
+                        for (int u = 0; u < RW; u++)
 #pragma unroll
-                            for (int q = 0; q < VEC; q++) {
-                                if (k0 + q < klim) {
-                                    const T x = dk && a.cjp ? conj_v(e[u][q]) : e[u][q];
+                            for (int q = 0; q < VEC; q++)
+                                if (dk && a.cjp) e[u][q] = conj_v(e[u][q]);
 #pragma unroll
-                                    for (int r = 0; r < NR; r++) acc[u][r] += x * vv[q][r];
-                                }
+                        for (int r = 0; r < NR; r++) {
+                            T v[VEC];
+                            const uint4 u4 = lds_u4(sv + (uint32_t)(r * vpitch + k0) * sizeof(T));
+                            memcpy(v, &u4, 16);
+#pragma unroll
+                            for (int u = 0; u < RW; u++) {
+                                const int klim = dk ? r0 + warp + FLOW_CWARPS * u + 1 : w;
+#pragma unroll
+                                for (int q = 0; q < VEC; q++)
+                                    if (k0 + q < klim) acc[u * NR + r] += e[u][q] * v[q];
                             }
                         }
                     }
                 }
+                // sums over the lanes: each step halves the values a lane carries (NA - 1 exchanges while
+                // more than one is left, instead of 5 NA), after which lane l holds value l >> SH
+                int cnt = NA;
 #pragma unroll
-                for (int u = 0; u < RW; u++)
+                for (int o = 16; o > 0; o >>= 1) {
+                    if (cnt > 1) {
+                        cnt >>= 1;
 #pragma unroll
-                    for (int r = 0; r < NR; r++)
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) acc[u][r] += shfl_xor_v(acc[u][r], o);
-                // lane u stores row warp + 8 u
-#pragma unroll
-                for (int u = 0; u < RW; u++) {
-                    const int i = warp + FLOW_CWARPS * u;
-                    if (lane == u && i < nr) {
-                        if (dk) {
-                            const int n = r0 + i;
-                            T d = T(1);
-                            if (a.ldl) {
-                                d = a.coef[q.aux + (int64_t)n * ld + n];
-                                if (a.cjp) d = conj_v(d);
+                        for (int x = 0; x < NA / 2; x++)
+                            if (x < cnt) {
+                                const bool up = (lane & o) != 0;
+                                const T send = up ? acc[x] : acc[x + cnt], keep = up ? acc[x + cnt] : acc[x];
+                                acc[x] = keep + shfl_xor_v(send, o);
                             }
-#pragma unroll
-                            for (int r = 0; r < NR; r++)
-                                a.Y[(int64_t)r * a.ldb + fc + n] = a.ldl ? acc[u][r] * d : acc[u][r];
-                        } else {
-                            const int grow = rowsm[s][i];
-#pragma unroll
-                            for (int r = 0; r < NR; r++) atomic_sub(&a.B[(int64_t)r * a.ldb + grow], acc[u][r]);
+                    } else {
+                        acc[0] += shfl_xor_v(acc[0], o);
+                    }
+                }
+                constexpr int SH = NA == 32 ? 0 : NA == 16 ? 1 : NA == 8 ? 2 : 3;
+                static_assert(NA == 32 || NA == 16 || NA == 8 || NA == 4, "one value per lane group");
+                const int u = (lane >> SH) / NR, r = (lane >> SH) % NR, i = warp + FLOW_CWARPS * u;
+                if ((lane & ((1 << SH) - 1)) == 0 && i < nr && r < a.nv) {
+                    if (dk) {
+                        const int n = r0 + i;
+                        T d = T(1);
+                        if (a.ldl) {
+                            d = a.coef[q.aux + (int64_t)n * ld + n];
+                            if (a.cjp) d = conj_v(d);
                         }
+                        a.Y[(int64_t)r * a.ldb + fc + n] = a.ldl ? acc[0] * d : acc[0];
+                    } else {
+                        atomic_sub(&a.B[(int64_t)r * a.ldb + rowsm[s][i]], acc[0]);
                     }
                 }
             } else {
@@ -498,15 +503,29 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_solve_flow(FlowArgs<T> a) {
                     for (int i = i0; i < nr; i++) {
                         T e = lds_t<T>(sP + (uint32_t)(i * ld + j) * sizeof(T));
                         if (kind == FLOW_O && a.cjp) e = conj_v(e);
+                        if constexpr (NR * sizeof(T) >= 16) {
+                            constexpr int VEC = 16 / sizeof(T);
 #pragma unroll
-                        for (int r = 0; r < NR; r++) sm[r] += e * lds_t<T>(sv + (uint32_t)(i * NR + r) * sizeof(T));
+                            for (int r = 0; r < NR; r += VEC) {
+                                T v[VEC];
+                                const uint4 u4 = lds_u4(sv + (uint32_t)(i * NR + r) * sizeof(T));
+                                memcpy(v, &u4, 16);
+#pragma unroll
+                                for (int x = 0; x < VEC; x++) sm[r + x] += e * v[x];
+                            }
+                        } else {
+#pragma unroll
+                            for (int r = 0; r < NR; r++) sm[r] += e * lds_t<T>(sv + (uint32_t)(i * NR + r) * sizeof(T));
+                        }
                     }
                     if (kind == FLOW_O) {
 #pragma unroll
-                        for (int r = 0; r < NR; r++) atomic_sub(&a.B[(int64_t)r * a.ldb + fc + j], sm[r]);
+                        for (int r = 0; r < NR; r++)
+                            if (r < a.nv) atomic_sub(&a.B[(int64_t)r * a.ldb + fc + j], sm[r]);
                     } else {
 #pragma unroll
-                        for (int r = 0; r < NR; r++) atomic_add(&a.Z[(int64_t)r * a.ldb + fc + j], sm[r]);
+                        for (int r = 0; r < NR; r++)
+                            if (r < a.nv) atomic_add(&a.Z[(int64_t)r * a.ldb + fc + j], sm[r]);
                     }
                 }
             }
@@ -543,16 +562,16 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_solve_flow(FlowArgs<T> a) {
             }
             last = __shfl_sync(0xffffffffu, last, 0);
             if (last) {
-                for (int e = lane; e < q.w * NR; e += 32) {
-                    const int j = e / NR, r = e - j * NR;
-                    const int64_t o = (int64_t)r * a.ldb + q.fc + j;
-                    if (FWD) {
-                        a.B[o] = ldcg_v(a.Y + o);
-                    } else {
-                        a.B[o] = ldcg_v(a.Z + o);
-                        a.Z[o] = T(0);
+                for (int r = 0; r < a.nv; r++)
+                    for (int j = lane; j < q.w; j += 32) {
+                        const int64_t o = (int64_t)r * a.ldb + q.fc + j;
+                        if (FWD) {
+                            a.B[o] = ldcg_v(a.Y + o);
+                        } else {
+                            a.B[o] = ldcg_v(a.Z + o);
+                            a.Z[o] = T(0);
+                        }
                     }
-                }
                 __syncwarp();
                 if (!FWD && lane == 0) {
                     __threadfence();
