@@ -203,6 +203,7 @@ struct pastix_gpu_s {
     // coeftab and of the inverses (3xTF32), one tensor map per (source cblk,
     // operand kind), split jobs {cblk, row, panel, -} per level
     bool tma = false;
+    bool forms_off = false;   // no room (or no tensor maps) for the LDL / complex planes
     DArr<float> d_hilo, d_ihilo;
     // 3xFP16 operands (mixed GEMM mode 3): FP16 hi / lo planes [2][h16_plane]
     // of the source matrices, per-row inverse scales, and per operand map its
@@ -212,7 +213,7 @@ struct pastix_gpu_s {
     DArr<float> d_hscale;
     DArr<int64_t> d_hoff, d_hsbase;
     int64_t h16_plane = 0;
-    // per task {target-row map base, A row-scale base, B row-scale base} and
+    // per task its target-row map's base, and
     // the target rows of the tensor-core update tasks (k_task_rowmap)
     DArr<int64_t> d_taux;
     DArr<int> d_tmap, d_tlist;
@@ -458,6 +459,7 @@ extern "C" int pastix_gpu_structure(pastix_gpu_t *ctx, int64_t n, int64_t cblknb
     }
     PGPU_CHECK(C.d_solve_chunks.upload(sch, s));
     C.plan_fact = -1;
+    C.forms_off = false;
     C.fact_done = -1;
     C.d_coef.release();
     PGPU_CHECK(cudaStreamSynchronize(s));
@@ -884,7 +886,12 @@ static int build_flow_plan(pastix_gpu_t &C, size_t esz, bool lu) {
 }
 
 static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
-    const bool use_tc = fp32 && !zc && tc_enabled(C) && (fmode == FM_POTRF || fmode == FM_GETRF);
+    // single precision: the large update and TRSM GEMMs on the tcgen05 tensor cores; the LDL and the
+    // complex forms only as 3xFP16 with pre-split operands (D and the complex product live in the planes)
+    const bool h16_forms = fp32 && mixed_gemm_mode(C) == MG_3XF16 && C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record &&
+                           C.tune[PGPU_TUNE_TC_TMA] != 0 && tensor_map_encoder() != nullptr && !C.forms_off;
+    const bool use_tc = fp32 && tc_enabled(C) && ((!zc && (fmode == FM_POTRF || fmode == FM_GETRF)) || h16_forms);
+    const int cs = zc ? 2 : 1;   // floats per element: the tensor-core tiles of complex tasks are real ones
     // real FP64: the large update and TRSM GEMMs on the FP64 tensor cores (DMMA),
     // planned like the single-precision tensor-core tiles (128 x 64 tiles)
     const bool use_dmma = !fp32 && !zc && C.tune[PGPU_TUNE_DMMA] != 0 && !C.record;
@@ -903,7 +910,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     const size_t esz = (fp32 ? 4 : 8) * (zc ? 2 : 1);
     const int fuse = tgemm ? std::min((int)C.tune[PGPU_TUNE_TRSM_GEMM_ROWS], fuse_rows_for(lu, esz))
                            : fuse_rows_for(lu, esz);
-    const bool tc_trsm = tgemm && ((fp32 && !zc && tc_enabled(C)) || use_dmma);
+    const bool tc_trsm = tgemm && ((fp32 && tc_enabled(C) && (!zc || h16_forms)) || use_dmma);
     std::vector<int2> invjobs;
     std::vector<int4> ttiles, tttiles;
     int64_t inv_elems = 0, scr_max = 0;
@@ -1001,7 +1008,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                     tasks.push_back(g);
                     const int bm = tc_trsm ? tbm : GEMM_TM, bn = tc_trsm ? tbn : GEMM_TN;
                     for (int tm = 0; tm < cdiv(h - w, bm); tm++)
-                        for (int tn = 0; tn < cdiv(w, bn); tn++)
+                        for (int tn = 0; tn < cdiv((tc_trsm ? cs : 1) * w, bn); tn++)
                             (tc_trsm ? tttiles : ttiles).push_back(make_int4(id, tm, tn, 0));
                 }
             } else if (h > fuse && h == w && tgemm) {
@@ -1023,11 +1030,11 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                     const int id = (int)tasks.size();
                     tasks.push_back(GemmTask{c, b, f, arow0, M, flags});
                     gflops += fma_flops * M * N * w;
-                    if ((use_tc || use_dmma) && tc_task(C, M, N, w)) {
-                        tcflops += 2.0 * M * N * w;
+                    if ((use_tc || use_dmma) && tc_task(C, M, cs * N, cs * w)) {
+                        tcflops += fma_flops * M * N * w;
                         for (int tm = 0; tm < cdiv(M, tbm); tm++)
-                            for (int tn = 0; tn < cdiv(N, tbn); tn++) {
-                                if ((flags & 8) && (int64_t)(tm + 1) * tbm <= (int64_t)tn * tbn) continue;
+                            for (int tn = 0; tn < cdiv(cs * N, tbn); tn++) {
+                                if ((flags & 8) && (int64_t)(tm + 1) * tbm <= (int64_t)tn * tbn / cs) continue;
                                 ltc[crit].push_back(make_int4(id, tm, tn, 0));
                             }
                         return;
@@ -1096,9 +1103,21 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
         std::vector<int> mapidx(C.cblknbr, -1);
         std::vector<int64_t> hoff, hsbase;
         int64_t hp = 0, sp = 0;
+        // a cblk whose rows go through the TRSM GEMM: the split before it takes the operands of that GEMM,
+        // its copy-back the updates' (all kinds of the others' are split at the end of their level)
+        auto tall = [&](int c) { return tgemm && C.height[c] > fuse && C.height[c] > C.width[c]; };
         auto needed = [&](int c, int kind) {
-            return kind == TMAP_L || (kind == TMAP_U && lu) || (kind == TMAP_I && C.invoff[c] >= 0) ||
-                   (kind == TMAP_I2 && lu && C.invoff[c] >= 0);
+            switch (kind) {
+            case TMAP_L: return true;
+            case TMAP_U: return lu || ldl;
+            case TMAP_I: return tall(c);
+            case TMAP_I2: return lu && tall(c);
+            case TMAP_BL: return zc;
+            default: return zc && lu;
+            }
+        };
+        auto map_rows = [&](int c, int kind) {
+            return (kind == TMAP_I || kind == TMAP_I2 ? C.width[c] : C.height[c]) * (kind >= TMAP_I ? cs : 1);
         };
         for (int l = 0; l < C.nlevels; l++)
             for (int q = C.lvl_ptr[l]; q < C.lvl_ptr[l + 1]; q++) {
@@ -1108,16 +1127,29 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 mapidx[c] = (int)hoff.size();
                 for (int kind = 0; kind < TMAP_KINDS; kind++) {
                     const bool nd = needed(c, kind);
-                    const int rows = kind < TMAP_I ? C.height[c] : w;
+                    const int rows = map_rows(c, kind);
                     hoff.push_back(nd ? hp : -1);
                     hsbase.push_back(nd ? sp : -1);
                     if (nd) {
-                        hp += round_up((int64_t)rows * ld16_of(w), 64);
+                        hp += round_up((int64_t)rows * ld16_of(cs * w), 64);
                         sp += rows;
                     }
                 }
             }
         C.h16_plane = round_up(std::max<int64_t>(hp, 64), 64);
+        if (zc || ldl) {
+            // (complex planes are three times the factor: where they do not fit beside it, FMA tiles)
+            size_t mfree = 0, mtotal = 0;
+            PGPU_CHECK(cudaMemGetInfo(&mfree, &mtotal));
+            auto more = [](size_t want, size_t have) { return want > have ? want : 0; };
+            const size_t need = more(4 * (size_t)C.h16_plane, C.d_h16.n * 2) +
+                                more((size_t)C.coefnbr * (lu ? 2 : 1) * esz, C.d_coef.n) +
+                                more((size_t)inv_elems * esz, C.d_inv.n) + more((size_t)scr_max * esz, C.d_scr.n);
+            if (need + need / 8 > mfree) {
+                C.forms_off = true;
+                return build_fact_plan(C, fmode, fp32, zc);
+            }
+        }
         if (C.d_h16.n < (size_t)(2 * C.h16_plane)) PGPU_CHECK(C.d_h16.alloc(2 * C.h16_plane));
         if (C.d_hscale.n < (size_t)std::max<int64_t>(sp, 1)) PGPU_CHECK(C.d_hscale.alloc(std::max<int64_t>(sp, 1)));
         std::vector<CUtensorMap> maps(hoff.size());
@@ -1131,11 +1163,14 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 for (int kind = 0; kind < TMAP_KINDS; kind++) {
                     const int mi = mapidx[c] + kind;
                     if (hoff[mi] < 0) continue;
-                    const int rows = kind < TMAP_I ? h : w;
-                    if (!encode_h16_map(&maps[mi], C.d_h16.p + hoff[mi], w, rows, ld16_of(w), C.h16_plane))
+                    if (!encode_h16_map(&maps[mi], C.d_h16.p + hoff[mi], cs * w, map_rows(c, kind), ld16_of(cs * w),
+                                        C.h16_plane))
                         C.tma = false;
                     // panels: their off-diagonal rows; inverses: all rows
-                    for (int r0 = kind < TMAP_I ? w : 0; r0 < rows; r0 += 32) split.push_back(make_int4(c, r0, kind, 0));
+                    const bool isinv = kind == TMAP_I || kind == TMAP_I2;
+                    if (tall(c) && !isinv && kind != TMAP_L && !(kind == TMAP_U && lu)) continue;   // the copy-back's
+                    for (int r0 = isinv ? 0 : w; r0 < (isinv ? w : h); r0 += 32)
+                        split.push_back(make_int4(c, r0, kind, 0));
                 }
             }
             C.split_ptr[l + 1] = (int)split.size();
@@ -1149,6 +1184,10 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             mapidx_h.swap(mapidx);
             hsbase_h.swap(hsbase);
         } else {
+            if (zc || ldl) {   // (their tiles have no other tensor-core kernel)
+                C.forms_off = true;
+                return build_fact_plan(C, fmode, fp32, zc);
+            }
             C.h16 = false;
             C.split_ptr.assign(C.nlevels + 1, 0);
         }
@@ -1275,7 +1314,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     for (const std::vector<int4> *lst : {&tctiles, &tttiles})
         for (const int4 &t : *lst) {
             const GemmTask &g = tasks[t.x];
-            const int N = (g.flags & 64) ? C.width[g.c] : C.blrow[g.b] - C.bfrow[g.b] + 1;
+            const int N = cs * ((g.flags & 64) ? C.width[g.c] : C.blrow[g.b] - C.bfrow[g.b] + 1);
             if ((int64_t)t.y * tbm >= g.M || (int64_t)t.z * tbn >= N ||
                 ((t.w & 1) && (int64_t)(t.y + 1) * tbm >= g.M)) {
                 fprintf(stderr, "pastix_gpu: tensor-core tile outside its task (plan error)\n");
@@ -1287,8 +1326,8 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     PGPU_CHECK(C.d_trsm.upload(trsm, s));
     PGPU_CHECK(C.d_tasks.upload(tasks, s));
     if (C.tma || use_dmma) {
-        // tensor-core tasks: target-row maps (built on the device) and scale bases
-        std::vector<int64_t> taux(3 * tasks.size(), 0);
+        // tensor-core tasks: target-row maps (built on the device)
+        std::vector<int64_t> taux(tasks.size(), 0);
         std::vector<char> is_tc(tasks.size(), 0);
         for (const int4 &t : tctiles) is_tc[t.x] = 1;
         std::vector<int> tlist;
@@ -1297,16 +1336,9 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             const GemmTask &g = tasks[i];
             const bool trsm = (g.flags & 64) != 0;
             if (is_tc[i] && !trsm) {
-                taux[3 * i] = rows;
+                taux[i] = rows;
                 rows += g.M;
                 tlist.push_back((int)i);
-            }
-            if (C.h16 && (is_tc[i] || trsm) && mapidx_h[g.c] >= 0) {
-                const int mb = mapidx_h[g.c];
-                const int ka = (g.flags & 1) ? TMAP_U : TMAP_L;
-                const int kb = trsm ? ((g.flags & 128) ? TMAP_I2 : TMAP_I) : ((g.flags & 2) ? TMAP_U : TMAP_L);
-                taux[3 * i + 1] = hsbase_h[mb + ka] + g.arow0;
-                taux[3 * i + 2] = hsbase_h[mb + kb] + (trsm ? 0 : C.browoff[g.b]);
             }
         }
         PGPU_CHECK(C.d_taux.upload(taux, s));
@@ -1316,34 +1348,37 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 const GemmTask &g = tasks[t.x];
                 const bool trsm = (g.flags & 64) != 0;
                 const int c = g.c, w = C.width[c];
-                const int N = trsm ? w : C.blrow[g.b] - C.bfrow[g.b] + 1;
+                const int N = cs * (trsm ? w : C.blrow[g.b] - C.bfrow[g.b] + 1);
                 const int i0 = t.y * TC_BM, j0 = t.z * TC_BN;
+                const int ka = ((g.flags & 1) || (ldl && !trsm)) ? TMAP_U : TMAP_L;
+                const int kb = trsm ? ((g.flags & 128) ? TMAP_I2 : TMAP_I)
+                                    : ((g.flags & 2) ? (zc ? TMAP_BU : TMAP_U) : (zc ? TMAP_BL : TMAP_L));
                 const int mb = mapidx_h[c];
                 TcDesc d;
                 std::memset(&d, 0, sizeof(d));
-                d.mapa = mb + ((g.flags & 1) ? TMAP_U : TMAP_L);
-                d.mapb = mb + (trsm ? ((g.flags & 128) ? TMAP_I2 : TMAP_I) : ((g.flags & 2) ? TMAP_U : TMAP_L));
+                d.mapa = mb + ka;
+                d.mapb = mb + kb;
                 d.rowa = g.arow0 + i0;
-                d.rowb = (trsm ? 0 : C.browoff[g.b]) + j0;
-                d.nk = cdiv(w, C.h16 ? 64 : TC_BK);
+                d.rowb = cs * (trsm ? 0 : C.browoff[g.b]) + j0;
+                d.nk = cdiv(cs * w, C.h16 ? 64 : TC_BK);
                 d.ncols = std::min(TC_BN, N - j0);
                 d.pair = t.w & 1;
-                d.flags = g.flags;
+                d.flags = g.flags | (zc ? TC_FLAG_CPLX : 0);
                 d.mrows = g.M - i0;
                 if (trsm) {
-                    d.ldo = C.ld[c];
-                    d.off = g.out + (int64_t)i0 * C.ld[c] + j0;
+                    d.ldo = cs * C.ld[c];
+                    d.off = cs * (g.out + (int64_t)i0 * C.ld[c]) + j0;
                 } else {
                     const int f = g.f;
-                    d.ldo = C.ld[f];
+                    d.ldo = cs * C.ld[f];
                     d.wf = C.width[f];
-                    d.tcol = C.bfrow[g.b] + j0 - C.fcol[f];
-                    d.off = ((g.flags & 4) ? C.coefnbr : 0) + C.coefoff[f];
-                    d.rmap = taux[3 * (size_t)t.x] + i0;
+                    d.tcol = cs * (C.bfrow[g.b] - C.fcol[f]) + j0;
+                    d.off = cs * (((g.flags & 4) ? C.coefnbr : 0) + C.coefoff[f]);
+                    d.rmap = taux[t.x] + i0;
                 }
                 if (C.h16) {
-                    d.sa = taux[3 * (size_t)t.x + 1] + i0;
-                    d.sb = taux[3 * (size_t)t.x + 2] + j0;
+                    d.sa = hsbase_h[mb + ka] + d.rowa;
+                    d.sb = hsbase_h[mb + kb] + d.rowb;
                 }
                 return d;
             };
@@ -1501,6 +1536,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
     PGPU_CHECK(cudaMemsetAsync(C.d_prog.p, 0, (size_t)(C.pr_counters + C.nlevels) * sizeof(int), s));
     // the Hermitian forms conjugate the L coefficients in the row solves
     constexpr bool CPX = is_cplx<T>::value;
+    constexpr bool F32 = sizeof(typename real_of<T>::type) == 4;   // factors whose GEMMs run on tcgen05
     auto ktrsm = (CPX && fm_conj(fmode)) ? k_trsm_rows<T, TRSM_TR, CPX> : k_trsm_rows<T, TRSM_TR, false>;
     PGPU_CHECK(cudaFuncSetAttribute(kpanel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
     PGPU_CHECK(cudaFuncSetAttribute(ktrsm, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
@@ -1509,7 +1545,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
     const bool split = (mixed_gemm_mode(C) == MG_3XTF32 || mixed_gemm_mode(C) == MG_3XF16);
     const bool persist = C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record;   // task timings need one tile per CTA
     int nsm = 148;
-    if constexpr (std::is_same<T, float>::value) {
+    if constexpr (F32) {
         PGPU_CHECK(cudaFuncSetAttribute(k_gemm_scatter_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         tc_smem_bytes<false>()));
         PGPU_CHECK(cudaFuncSetAttribute(k_gemm_scatter_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1554,17 +1590,19 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
     }
     // hi / lo split of the level's tensor-core source rows (before their first use as TMA operands)
     auto split_level = [&](int l) {
-        if constexpr (std::is_same<T, float>::value) {
+        if constexpr (F32) {
             const int nsp = C.split_ptr[l + 1] - C.split_ptr[l];
             if (C.tma && C.h16 && nsp) {
-                k_split_rows_h16<<<nsp, 256, 0, s>>>(C.meta, C.d_split.p + C.split_ptr[l], coefL, coefU,
-                                                     reinterpret_cast<const float *>(C.d_inv.p), C.d_h16.p,
-                                                     C.h16_plane, C.d_hscale.p, C.d_hoff.p, C.d_hsbase.p,
-                                                     C.d_mapidx.p);
+                k_split_rows_h16<T><<<nsp, 256, 0, s>>>(C.meta, C.d_split.p + C.split_ptr[l], coefL, coefU,
+                                                        reinterpret_cast<const T *>(C.d_inv.p), C.d_h16.p,
+                                                        C.h16_plane, C.d_hscale.p, C.d_hoff.p, C.d_hsbase.p,
+                                                        C.d_mapidx.p, fm_ldl(fmode) ? 1 : 0,
+                                                        (CPX && fm_conj(fmode)) ? 1 : 0);
                 nl++;
             } else if (C.tma && nsp) {
-                k_split_rows<<<nsp, 256, 0, s>>>(C.meta, C.d_split.p + C.split_ptr[l], coefL, coefU, C.d_hilo.p,
-                                                 C.hilo_plane, C.coefnbr);
+                if constexpr (!CPX)
+                    k_split_rows<<<nsp, 256, 0, s>>>(C.meta, C.d_split.p + C.split_ptr[l], coefL, coefU, C.d_hilo.p,
+                                                     C.hilo_plane, C.coefnbr);
                 nl++;
             }
         }
@@ -1595,6 +1633,17 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                 PGPU_CHECK(lt.mark(PH_TC));
                 k_gemm_scatter_dmma<<<ntc, DG_THREADS, dg_smem_bytes(), st>>>(
                     C.meta, C.d_tctiles.p + c0, C.d_tasks.p, coefL, coefU, nullptr, nullptr, C.d_tmap.p, C.d_taux.p);
+                if (la) PGPU_CHECK(lt.mark(PH_END));
+                nl++;
+                ngemm++;
+            }
+        }
+        if constexpr (F32 && CPX) {
+            if (ntc) {   // (planned for the 3xFP16 operands only)
+                PGPU_CHECK(lt.mark(PH_TC));
+                k_gemm_scatter_tc_tma<true, true><<<std::min(ntc, gcap), TMA_THREADS, tma_smem_bytes<true>(), st>>>(
+                    C.d_tcdesc.p + c0, ntc, reinterpret_cast<float *>(coefL), C.d_status.p, nullptr, C.d_tmaps.p,
+                    C.d_tmap.p, C.d_hscale.p);
                 if (la) PGPU_CHECK(lt.mark(PH_END));
                 nl++;
                 ngemm++;
@@ -1722,6 +1771,15 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                     nl++;
                 }
             }
+            if constexpr (F32 && CPX) {
+                const int ntc = C.tttile_ptr[l + 1] - C.tttile_ptr[l];
+                if (ntc) {
+                    k_gemm_scatter_tc_tma<true, true><<<std::min(ntc, nsm), TMA_THREADS, tma_smem_bytes<true>(), s>>>(
+                        C.d_ttdesc.p + C.tttile_ptr[l], ntc, reinterpret_cast<float *>(coefL), C.d_status.p,
+                        reinterpret_cast<float *>(scr), C.d_tmaps.p, C.d_tmap.p, C.d_hscale.p);
+                    nl++;
+                }
+            }
             if constexpr (std::is_same<T, float>::value) {
                 const int ntc = C.tttile_ptr[l + 1] - C.tttile_ptr[l];
                 if (ntc) {
@@ -1745,12 +1803,13 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                 }
             }
             bool copied = false;
-            if constexpr (std::is_same<T, float>::value) {
+            if constexpr (F32) {
                 if (C.tma && C.h16) {
                     if (ntr)
-                        k_trsm_copyback_h16<<<ntr, 256, 0, s>>>(C.meta, C.d_trsm.p + C.trsm_ptr[l], C.d_scroff.p,
-                                                                scr, coefL, coefU, C.d_h16.p, C.h16_plane,
-                                                                C.d_hscale.p, C.d_hoff.p, C.d_hsbase.p, C.d_mapidx.p);
+                        k_trsm_copyback_h16<T><<<ntr, 256, 0, s>>>(
+                            C.meta, C.d_trsm.p + C.trsm_ptr[l], C.d_scroff.p, scr, coefL, coefU, C.d_h16.p,
+                            C.h16_plane, C.d_hscale.p, C.d_hoff.p, C.d_hsbase.p, C.d_mapidx.p,
+                            fm_ldl(fmode) ? 1 : 0, (CPX && fm_conj(fmode)) ? 1 : 0);
                     copied = true;
                 }
             }

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(DG_THREADS, 2)
     // target row of each of this thread's output rows (one row-map load each)
     int trow[4][2];
     {
-        const int64_t tb = trsm ? 0 : taux[3 * (int64_t)tl.x];
+        const int64_t tb = trsm ? 0 : taux[tl.x];
 #pragma unroll
         for (int mi = 0; mi < 4; mi++) {
             const int r = wm * 32 + mi * 8 + (lane >> 2);

@@ -44,8 +44,10 @@ namespace pgpu {
 constexpr int TMA_THREADS = 320, TMA_EPI_WARPS = 8;
 constexpr int TMA_PROD_WARP = 4, TMA_MMA_WARP = 5;
 constexpr int TMA_EPI_BYTES = TMA_EPI_WARPS * 32 * 32 * 4;   // a swizzled 32 x 32 float buffer per warp
-// operand maps per cblk: L panel, U panel (LU), first / second diagonal-block inverse
-enum { TMAP_L = 0, TMAP_U = 1, TMAP_I = 2, TMAP_I2 = 3, TMAP_KINDS = 4 };
+// operand maps per cblk: L panel, U panel (LU; LDL: the L rows times D), first / second diagonal-block
+// inverse, and in complex arithmetic the L / U panels as B operands (two real rows per row, see below)
+enum { TMAP_L = 0, TMAP_U = 1, TMAP_I = 2, TMAP_I2 = 3, TMAP_BL = 4, TMAP_BU = 5, TMAP_KINDS = 6 };
+constexpr int TC_FLAG_CPLX = 256;   // TcDesc::flags: real and imaginary parts are neighbouring columns
 
 // A stage holds two A tiles (a pair of 128-row tiles of one task sharing the
 // B tile) and the B tile; hi and lo planes each for 3xTF32.
@@ -104,6 +106,16 @@ __device__ __forceinline__ TcDesc tc_desc_load(const TcDesc *p) {
 // covers K = 16.  The epilogue multiplies the accumulator by the rows'
 // inverse scales 2^-e_a 2^-e_b (hscale, one float per source row; hsbase
 // gives each operand map's first row there), exact powers of two.
+//
+// Complex C = A op(B)^t as a real product of twice the columns and depth: a
+// row of A is its interleaved (re, im) pairs as they lie in the panel; a row
+// of B becomes two, whose products with it are the real and the imaginary
+// part -- (re, -im) and (im, re), or for op = conj (re, im) and (-im, re) --
+// so that neighbouring columns of the accumulator are re and im, as in the
+// target panel, and the epilogue is the real one.  The planes of a complex
+// panel are three times its size, written once per cblk.  Measured on one
+// B200 against the FMA tiles: 60^3 complex64 LDL^h factorization 59.4 -> 18.7
+// ms, 53x49x61 real LDL^t 9.9 -> 5.7 ms.
 template <bool SPLIT, bool F16 = false>
 __global__ void __launch_bounds__(TMA_THREADS, 1)
     k_gemm_scatter_tc_tma(const TcDesc *__restrict__ desc, int ntiles, float *__restrict__ coefL, Status *st,
@@ -315,6 +327,7 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
             const int ldf = v.ldo, wf = v.wf;
             const int tcol0 = v.tcol;
             const bool lower_only = (v.flags & 8) != 0;
+            const int csh = (v.flags & TC_FLAG_CPLX) ? 1 : 0;
             // the update subtracts: the sign rides on the row scale
             const float sgn = trsm ? 1.f : -1.f;
             for (int h = 0; h < nh; h++)
@@ -379,7 +392,7 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
 #pragma unroll
                                 for (int u = 0; u < 4; u++) {
                                     const int jj = j0 + u, tc = a0 + 4 * g + u;
-                                    const bool ok = jj >= 0 && jj < nvalid && !(lower_only && t2 < wf && tc > t2);
+                                    const bool ok = jj >= 0 && jj < nvalid && !(lower_only && t2 < wf && (tc >> csh) > t2);
                                     a[u] = ok ? a[u] : 0.f;
                                     any |= ok;
                                 }
@@ -449,167 +462,195 @@ __global__ void k_split_rows(Meta m, const int4 *__restrict__ jobs, const float 
 // e = 0).  The row's stored scale is 2^-e, which the GEMM epilogue applies.
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
 
-// One warp splits one row of w floats (src 16-byte aligned when w >= 4):
-// optional FP32 copy to dst, hi / lo halves at hi and hi + hplane, the
-// inverse scale at *sc.
-__device__ __forceinline__ void split_row_h16(const float *__restrict__ src, int w, float *__restrict__ dst,
-                                              __half *__restrict__ hi, int64_t hplane, float *__restrict__ sc,
-                                              int lane) {
-    const int wv = w >> 2;
-    constexpr int RV = 4;   // rows of up to 32 RV float4 stay in registers: read once, all loads in flight
-    if (wv <= 32 * RV) {
-        float4 x[RV];
-        float mx = 0.f;
+// One warp splits one row of nf floats (complex: interleaved parts; src 16-byte
+// aligned, padded to a multiple of 4): optionally times dsc (one factor per
+// matrix column), an FP32 copy to dst, hi / lo halves at ha and ha + hplane
+// (an A operand, or real B) with the inverse scale at *sa, and (complex) the
+// two rows of a B operand at hb and hb + ldb with their scales at sb[0 .. 1].
+template <typename T>
+__device__ __forceinline__ void split_row_h16(const T *__restrict__ src_t, int nf, const T *dsc, T *__restrict__ dst_t,
+                                              __half *__restrict__ ha, float *__restrict__ sa,
+                                              __half *__restrict__ hb, int ldb, float *__restrict__ sb, bool conjb,
+                                              int64_t hplane, int lane) {
+    constexpr bool CX = is_cplx<T>::value;
+    constexpr int RV = CX ? 8 : 4;   // the whole row in registers (at most 400 columns): read once, all loads in flight
+    const float *src = reinterpret_cast<const float *>(src_t);
+    float *dst = reinterpret_cast<float *>(dst_t);
+    const int nq = (nf + 3) >> 2;
+    float x[RV][4];
+    float mx = 0.f;
+#pragma unroll
+    for (int u = 0; u < RV; u++) {
+        const int q = lane + 32 * u;
+        float4 v = q < nq ? __ldg(reinterpret_cast<const float4 *>(src) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[u][0] = v.x; x[u][1] = v.y; x[u][2] = v.z; x[u][3] = v.w;
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (4 * q + e >= nf) x[u][e] = 0.f;
+    }
+    if (dsc) {
 #pragma unroll
         for (int u = 0; u < RV; u++) {
             const int q = lane + 32 * u;
-            x[u] = q < wv ? __ldg(reinterpret_cast<const float4 *>(src) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        const int jt = 4 * wv + lane;   // the tail (w % 4 columns), one per lane
-        const float xt = jt < w ? src[jt] : 0.f;
+            if (q >= nq) continue;
+            if constexpr (CX) {
 #pragma unroll
-        for (int u = 0; u < RV; u++)
-            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
-        mx = fmaxf(mx, fabsf(xt));
+                for (int e = 0; e < 4; e += 2)
+                    if (4 * q + e < nf) {
+                        const T y = T(x[u][e], x[u][e + 1]) * dsc[2 * q + e / 2];
+                        x[u][e] = y.re;
+                        x[u][e + 1] = y.im;
+                    }
+            } else {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        int e = 0;
-        if (mx > 0.f) {
-            const int E = ((__float_as_int(mx) >> 23) & 0xff) - 127;
-            e = max(-126, min(126, 14 - E));
-        }
-        const float s = pow2f(e);
-        if (lane == 0) *sc = pow2f(-e);
-        __half *lo = hi + hplane;
-#pragma unroll
-        for (int u = 0; u < RV; u++) {
-            const int q = lane + 32 * u;
-            if (q < wv) {
-                if (dst) reinterpret_cast<float4 *>(dst)[q] = x[u];
-                const float y[4] = {x[u].x * s, x[u].y * s, x[u].z * s, x[u].w * s};
-                __half h[4], l[4];
-#pragma unroll
-                for (int v = 0; v < 4; v++) {
-                    h[v] = __float2half_rn(y[v]);
-                    l[v] = __float2half_rn(y[v] - __half2float(h[v]));
-                }
-                reinterpret_cast<__half2 *>(hi)[2 * q] = __halves2half2(h[0], h[1]);
-                reinterpret_cast<__half2 *>(hi)[2 * q + 1] = __halves2half2(h[2], h[3]);
-                reinterpret_cast<__half2 *>(lo)[2 * q] = __halves2half2(l[0], l[1]);
-                reinterpret_cast<__half2 *>(lo)[2 * q + 1] = __halves2half2(l[2], l[3]);
+                for (int e = 0; e < 4; e++)
+                    if (4 * q + e < nf) x[u][e] *= dsc[4 * q + e];
             }
         }
-        if (jt < w) {
-            if (dst) dst[jt] = xt;
-            const float y = xt * s;
-            const __half h = __float2half_rn(y);
-            hi[jt] = h;
-            lo[jt] = __float2half_rn(y - __half2float(h));
-        }
-        return;
     }
-    float mx = 0.f;
-    for (int q = lane; q < wv; q += 32) {
-        const float4 x = reinterpret_cast<const float4 *>(src)[q];
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-    }
-    for (int j = 4 * wv + lane; j < w; j += 32) mx = fmaxf(mx, fabsf(src[j]));
+#pragma unroll
+    for (int u = 0; u < RV; u++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) mx = fmaxf(mx, fabsf(x[u][e]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    int e = 0;
+    int ex = 0;
     if (mx > 0.f) {
         const int E = ((__float_as_int(mx) >> 23) & 0xff) - 127;
-        e = max(-126, min(126, 14 - E));
+        ex = max(-126, min(126, 14 - E));
     }
-    const float s = pow2f(e);
-    if (lane == 0) *sc = pow2f(-e);
-    __half *lo = hi + hplane;
-    for (int q = lane; q < wv; q += 32) {
-        const float4 x = reinterpret_cast<const float4 *>(src)[q];
-        if (dst) reinterpret_cast<float4 *>(dst)[q] = x;
-        const float y[4] = {x.x * s, x.y * s, x.z * s, x.w * s};
-        __half h[4], l[4];
+    const float s = pow2f(ex);
+    if (lane == 0) {
+        if (ha) *sa = pow2f(-ex);
+        if (CX && hb) sb[0] = sb[1] = pow2f(-ex);
+    }
+    auto put = [&](__half *row, int q, __half a, __half b, __half c, __half d) {
+        __half2 v[2] = {__halves2half2(a, b), __halves2half2(c, d)};
+        uint2 w;
+        memcpy(&w, v, 8);
+        reinterpret_cast<uint2 *>(row)[q] = w;
+    };
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            h[u] = __float2half_rn(y[u]);
-            l[u] = __float2half_rn(y[u] - __half2float(h[u]));
+    for (int u = 0; u < RV; u++) {
+        const int q = lane + 32 * u;
+        if (q < nq) {
+            if (dst) reinterpret_cast<float4 *>(dst)[q] = make_float4(x[u][0], x[u][1], x[u][2], x[u][3]);
+            __half h[4], l[4];
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const float y = x[u][v] * s;
+                h[v] = __float2half_rn(y);
+                l[v] = __float2half_rn(y - __half2float(h[v]));
+            }
+            if (ha) {
+                put(ha, q, h[0], h[1], h[2], h[3]);
+                put(ha + hplane, q, l[0], l[1], l[2], l[3]);
+            }
+            if (CX && hb) {
+                __half *b1 = hb + ldb;
+                if (conjb) {
+                    put(hb, q, h[0], h[1], h[2], h[3]);
+                    put(hb + hplane, q, l[0], l[1], l[2], l[3]);
+                    put(b1, q, __hneg(h[1]), h[0], __hneg(h[3]), h[2]);
+                    put(b1 + hplane, q, __hneg(l[1]), l[0], __hneg(l[3]), l[2]);
+                } else {
+                    put(hb, q, h[0], __hneg(h[1]), h[2], __hneg(h[3]));
+                    put(hb + hplane, q, l[0], __hneg(l[1]), l[2], __hneg(l[3]));
+                    put(b1, q, h[1], h[0], h[3], h[2]);
+                    put(b1 + hplane, q, l[1], l[0], l[3], l[2]);
+                }
+            }
         }
-        reinterpret_cast<__half2 *>(hi)[2 * q] = __halves2half2(h[0], h[1]);
-        reinterpret_cast<__half2 *>(hi)[2 * q + 1] = __halves2half2(h[2], h[3]);
-        reinterpret_cast<__half2 *>(lo)[2 * q] = __halves2half2(l[0], l[1]);
-        reinterpret_cast<__half2 *>(lo)[2 * q + 1] = __halves2half2(l[2], l[3]);
-    }
-    for (int j = 4 * wv + lane; j < w; j += 32) {
-        const float x = src[j];
-        if (dst) dst[j] = x;
-        const float y = x * s;
-        const __half h = __float2half_rn(y);
-        hi[j] = h;
-        lo[j] = __float2half_rn(y - __half2float(h));
     }
 }
 
 // Target rows of the tensor-core update tasks, once per plan: for task
 // tlist[blockIdx.x] and each row i of its M rows, the panel row of the facing
 // cblk that source row arow0 + i lands in (kernels/core_zgemmsp.c:170-250
-// walks the facing blocks for this).  tmap[taux[3 task] + i].
+// walks the facing blocks for this).  tmap[taux[task] + i].
 __global__ void k_task_rowmap(Meta m, const GemmTask *__restrict__ tasks, const int *__restrict__ tlist,
                               const int64_t *__restrict__ taux, int *__restrict__ tmap) {
     const int id = tlist[blockIdx.x];
     const GemmTask t = tasks[id];
-    const int64_t base = taux[3 * (int64_t)id];
+    const int64_t base = taux[id];
     const int *rows = m.rowidx + m.rowbase[t.c] + t.arow0;
     for (int i = threadIdx.x; i < t.M; i += blockDim.x) tmap[base + i] = panel_row_of(m, t.f, rows[i]);
 }
 
 // Layout of the FP16 planes: per operand map (mapidx[c] + kind) the first
-// element in the planes (hoff, rows of ld16 = round_up(w_c, 8) halves) and the
-// first row in hscale (hsbase).
-__host__ __device__ inline int ld16_of(int w) { return (w + 7) & ~7; }
+// element in the planes (hoff, rows of ld16 halves, a multiple of 8 that holds
+// the row's floats) and the first row in hscale (hsbase).
+__host__ __device__ inline int ld16_of(int nf) { return (nf + 7) & ~7; }
+constexpr int H16_MAXW = 400;   // widest cblk (pastix_gpu_structure)
+
+// The pivots of cblk c (LDL: diagonal of its panel) into shared memory.
+template <typename T>
+__device__ __forceinline__ void load_pivots(const T *__restrict__ panel, int w, int ld, T *ds) {
+    for (int j = threadIdx.x; j < w; j += blockDim.x) ds[j] = panel[(int64_t)j * ld + j];
+}
 
 // Split jobs {cblk, first row, kind (TMAP_*), -}: rows [r0, r0 + 32) of the
-// source matrix of that kind (L / U panel rows, or the rows of the first /
-// second diagonal-block inverse), one warp per row.
+// source matrix of that kind (L / U panel rows, LDL: L times D for TMAP_U, or
+// the rows of the first / second diagonal-block inverse), one warp per row.
+template <typename T>
 __global__ void __launch_bounds__(256) k_split_rows_h16(Meta m, const int4 *__restrict__ jobs,
-                                                        const float *__restrict__ coefL,
-                                                        const float *__restrict__ coefU,
-                                                        const float *__restrict__ inv, __half *__restrict__ h16,
+                                                        const T *__restrict__ coefL, const T *__restrict__ coefU,
+                                                        const T *__restrict__ inv, __half *__restrict__ h16,
                                                         int64_t hplane, float *__restrict__ hscale,
                                                         const int64_t *__restrict__ hoff,
                                                         const int64_t *__restrict__ hsbase,
-                                                        const int *__restrict__ mapidx) {
+                                                        const int *__restrict__ mapidx, int ldl, int cj) {
+    constexpr bool CX = is_cplx<T>::value;
+    __shared__ __align__(16) unsigned char ds_raw[H16_MAXW * sizeof(T)];
+    T *ds = reinterpret_cast<T *>(ds_raw);
     const int4 jb = jobs[blockIdx.x];
     const int c = jb.x, r0 = jb.y, kind = jb.z;
-    const int w = m.width[c], ld = m.ld[c], l16 = ld16_of(w);
-    const int rows = kind < TMAP_I ? m.height[c] : w;
-    const float *src = kind == TMAP_L ? coefL + m.coefoff[c]
-                       : kind == TMAP_U ? coefU + m.coefoff[c]
-                                        : inv + m.invoff[c] + (kind == TMAP_I2 ? inv_span(w, ld) : 0);
+    const int w = m.width[c], ld = m.ld[c], nf = CX ? 2 * w : w, l16 = ld16_of(nf);
+    const bool isinv = kind == TMAP_I || kind == TMAP_I2, upper = kind == TMAP_U || kind == TMAP_BU;
+    const int rows = isinv ? w : m.height[c];
+    const T *src = isinv ? inv + m.invoff[c] + (kind == TMAP_I2 ? inv_span(w, ld) : 0)
+                         : ((upper && !ldl) ? coefU : coefL) + m.coefoff[c];
     const int mi = mapidx[c] + kind;
+    const bool pair = CX && kind >= TMAP_I;   // a B operand of complex data
+    const T *dsc = nullptr;
+    if (ldl && kind == TMAP_U) {
+        load_pivots(coefL + m.coefoff[c], w, ld, ds);
+        __syncthreads();
+        dsc = ds;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r1 = min(r0 + 32, rows);
-    for (int i = r0 + warp; i < r1; i += blockDim.x >> 5)
-        split_row_h16(src + (int64_t)i * ld, w, nullptr, h16 + hoff[mi] + (int64_t)i * l16, hplane,
-                      hscale + hsbase[mi] + i, lane);
+    for (int i = r0 + warp; i < r1; i += blockDim.x >> 5) {
+        const int row = pair ? 2 * i : i;
+        __half *h = h16 + hoff[mi] + (int64_t)row * l16;
+        float *sc = hscale + hsbase[mi] + row;
+        split_row_h16<T>(src + (int64_t)i * ld, nf, dsc, nullptr, pair ? nullptr : h, sc, pair ? h : nullptr, l16, sc,
+                         cj && !isinv, hplane, lane);
+    }
 }
 
 // TRSM copy-back with the FP16 split: rows [r0, r0 + 32) of the level's
 // TRSM output (chunks {cblk, r0, side, -} as k_trsm_copyback) into the panel
-// and, when the cblk is a tensor-core source, into its FP16 planes.
+// and, when the cblk is a tensor-core source, into the FP16 planes its
+// updates read.
+template <typename T>
 __global__ void __launch_bounds__(256) k_trsm_copyback_h16(Meta m, const int4 *__restrict__ chunks,
                                                            const int64_t *__restrict__ scroff,
-                                                           const float *__restrict__ scr, float *__restrict__ coefL,
-                                                           float *__restrict__ coefU, __half *__restrict__ h16,
+                                                           const T *__restrict__ scr, T *__restrict__ coefL,
+                                                           T *__restrict__ coefU, __half *__restrict__ h16,
                                                            int64_t hplane, float *__restrict__ hscale,
                                                            const int64_t *__restrict__ hoff,
                                                            const int64_t *__restrict__ hsbase,
-                                                           const int *__restrict__ mapidx) {
+                                                           const int *__restrict__ mapidx, int ldl, int cj) {
+    constexpr bool CX = is_cplx<T>::value;
+    __shared__ __align__(16) unsigned char ds_raw[H16_MAXW * sizeof(T)];
+    T *ds = reinterpret_cast<T *>(ds_raw);
     const int4 ch = chunks[blockIdx.x];
     const int c = ch.x, r0 = ch.y;
-    const int w = m.width[c], h = m.height[c], ld = m.ld[c], l16 = ld16_of(w);
+    const int w = m.width[c], h = m.height[c], ld = m.ld[c], nf = CX ? 2 * w : w, l16 = ld16_of(nf);
     const int nr = min(32, h - r0);
-    const float *src = scr + scroff[c] + (ch.z ? inv_span(h - w, ld) : 0) + (int64_t)(r0 - w) * ld;
-    float *dst = (ch.z ? coefU : coefL) + m.coefoff[c] + (int64_t)r0 * ld;
+    const T *src = scr + scroff[c] + (ch.z ? inv_span(h - w, ld) : 0) + (int64_t)(r0 - w) * ld;
+    T *dst = (ch.z ? coefU : coefL) + m.coefoff[c] + (int64_t)r0 * ld;
     const int mb = mapidx[c];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (mb < 0) {   // not a tensor-core source: the FP32 rows only
@@ -619,10 +660,23 @@ __global__ void __launch_bounds__(256) k_trsm_copyback_h16(Meta m, const int4 *_
         }
         return;
     }
-    const int mi = mb + (ch.z ? TMAP_U : TMAP_L);
-    for (int i = warp; i < nr; i += blockDim.x >> 5)
-        split_row_h16(src + (int64_t)i * ld, w, dst + (int64_t)i * ld, h16 + hoff[mi] + (int64_t)(r0 + i) * l16,
-                      hplane, hscale + hsbase[mi] + r0 + i, lane);
+    if (ldl) {
+        load_pivots(coefL + m.coefoff[c], w, ld, ds);
+        __syncthreads();
+    }
+    const int ka = mb + (ch.z ? TMAP_U : TMAP_L), kb = mb + (ch.z ? TMAP_BU : TMAP_BL);
+    const bool rowsa = !(CX && ldl);   // (complex LDL: the updates read L D and the B rows only)
+    for (int i = warp; i < nr; i += blockDim.x >> 5) {
+        const T *row = src + (int64_t)i * ld;
+        split_row_h16<T>(row, nf, nullptr, dst + (int64_t)i * ld,
+                         rowsa ? h16 + hoff[ka] + (int64_t)(r0 + i) * l16 : nullptr,
+                         rowsa ? hscale + hsbase[ka] + r0 + i : nullptr,
+                         CX ? h16 + hoff[kb] + (int64_t)(2 * (r0 + i)) * l16 : nullptr, l16,
+                         CX ? hscale + hsbase[kb] + 2 * (r0 + i) : nullptr, cj, hplane, lane);
+        if (ldl)
+            split_row_h16<T>(row, nf, ds, nullptr, h16 + hoff[mb + TMAP_U] + (int64_t)(r0 + i) * l16,
+                             hscale + hsbase[mb + TMAP_U] + r0 + i, nullptr, 0, nullptr, false, hplane, lane);
+    }
 }
 
 }  // namespace pgpu

@@ -1,0 +1,91 @@
+"""Tensor-core updates of the LDL and complex forms,
+against the numpy restatement."""
+import numpy as np
+import pytest
+
+from oracle.restate import sopalin_np as NP
+from pastix_b200 import analysis
+from pastix_b200 import matrices as M
+
+
+def _phased(A, seed):
+    """Complex general matrix with A's pattern and magnitudes."""
+    A.values = A.values * np.exp(0.3j * np.random.default_rng(seed).standard_normal(A.values.size))
+    return A
+
+
+def _csym(A, seed):
+    """Complex symmetric matrix, diagonally dominant as A is."""
+    A.values = A.values * (1 + 0.05j * np.random.default_rng(seed).standard_normal(A.values.size))
+    return A
+
+
+RNG = np.random.default_rng
+CASES = [
+    ("potrf", lambda: M.diffusion_lognormal(20, 17, 19, 1.0, RNG(2))),
+    ("sytrf", lambda: M.diffusion_lognormal(20, 17, 19, 1.0, RNG(2))),
+    ("getrf", lambda: M.convdiff_upwind(20, 17, 19, 10.0)),
+    ("potrf", lambda: M.magnetic_laplacian(15, 14, 16, -0.5, RNG(3))),
+    ("hetrf", lambda: M.magnetic_laplacian(15, 14, 16, 0.5, RNG(3))),
+    ("sytrf", lambda: _csym(M.diffusion_lognormal(15, 14, 16, 1.0, RNG(4)), 5)),
+    ("getrf", lambda: _phased(M.convdiff_upwind(15, 14, 16, 10.0), 6)),
+    ("sytrf", lambda: M.diffusion_lognormal(63, 50, 1, 0.5, RNG(7))),
+]
+IDS = ["potrf", "sytrf", "getrf", "potrf_z", "hetrf_z", "sytrf_z", "getrf_z", "sytrf_2d"]
+
+
+def _error(A, st, fact, L, U):
+    lay = NP.Layout(st["cblktab"], st["bloktab"])
+    L0, U0 = NP.fillin(lay, A, st["permtab"], lu=fact == "getrf")
+    NP.factorize(lay, L0, U0, fact, 0.0)
+    mask = np.ones(lay.off[-1], bool)
+    if fact != "getrf":
+        for c in range(lay.cblknbr):
+            k = int(lay.width[c])
+            lay.panel(mask, c)[:k, :] &= np.tril(np.ones((k, k), bool))
+    err = np.linalg.norm((L - L0)[mask]) / np.linalg.norm(L0[mask])
+    if fact == "getrf":
+        for c in range(lay.cblknbr):
+            lay.panel(mask, c)[:int(lay.width[c]), :] = False
+        err = max(err, np.linalg.norm((U - U0)[mask]) / np.linalg.norm(U0[mask]))
+    return err
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mixed", [True], ids=["mixed"])
+@pytest.mark.parametrize("fact,make", CASES, ids=IDS)
+def test_tensor_core_forms_match_restatement(fact, make, mixed):
+    """Factors as close to the 64-bit restatement as the FMA tiles' (the tensor-core sums round less
+    often), and the tensor cores carry the updates."""
+    from pastix_b200 import autotune as AT
+    from pastix_b200 import gpu as G
+    A = make()
+    st = analysis.analyze(A)
+    errs = []
+    for tc in (True, False):
+        s = G.Solver()
+        s.set_iparm(G.IPARM_FACTORIZATION, G.FACT[fact])
+        s.set_iparm(G.IPARM_MIXED, int(mixed))
+        s.set_structure(st)
+        s.set_spm(A)
+        if not tc:
+            AT.set_knob(s, "mixed_gemm", 0)
+            AT.set_knob(s, "dmma", 0)
+        try:
+            s.numfact(A.values)
+        except G.PastixGpuError as e:
+            s.close()
+            if e.code == 3:
+                pytest.skip("complex128 LU blocks this wide are not provided")
+            raise
+        stats = s.stats()
+        if tc and A.grid[2] > 1:
+            assert stats["tc_flops"] > 0.3 * stats["gemm_flops"] and stats["tc_timeouts"] == 0
+        L, U = s.coeftab()
+        errs.append(_error(A, st, fact, L, U))
+        s.close()
+    # unit roundoff times a few: diagonally dominant or of bounded growth; no worse than the FMA tiles
+    # beyond the spread between two summation orders
+    u = 2.0 ** (-24 if mixed else -53)
+    assert errs[0] <= 32 * u
+    assert errs[0] <= 1.5 * errs[1] + u / 4
