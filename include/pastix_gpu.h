@@ -273,7 +273,7 @@ PASTIX_GPU_API int pastix_gpu_phase_log( pastix_gpu_t *ctx, int64_t *count, int6
  *                             panel and loaded by TMA; 0: 3xTF32 split by producer warps per tile
  *   PGPU_TUNE_TC_PAIR_MIN     TMA kernel: fewest tiles in a launch for pairing 128-row
  *                             tiles that share their B tile (-1, default: 2 per SM)
- *   PGPU_TUNE_DMMA            1 (default): real FP64 update / TRSM GEMMs large enough
+ *   PGPU_TUNE_DMMA            1 (default): FP64 update / TRSM GEMMs large enough
  *                             for a 128 x 64 tile on the FP64 tensor cores (DMMA); 0: FMA tiles
  *   PGPU_TUNE_SOLVE_FLOW      1 (default): runs of solve levels whose cblks all hold a
  *                             diagonal-block inverse go through one dataflow launch per

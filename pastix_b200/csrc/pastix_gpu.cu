@@ -892,9 +892,9 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                            C.tune[PGPU_TUNE_TC_TMA] != 0 && tensor_map_encoder() != nullptr && !C.forms_off;
     const bool use_tc = fp32 && tc_enabled(C) && ((!zc && (fmode == FM_POTRF || fmode == FM_GETRF)) || h16_forms);
     const int cs = zc ? 2 : 1;   // floats per element: the tensor-core tiles of complex tasks are real ones
-    // real FP64: the large update and TRSM GEMMs on the FP64 tensor cores (DMMA),
+    // FP64: the large update and TRSM GEMMs on the FP64 tensor cores (DMMA),
     // planned like the single-precision tensor-core tiles (128 x 64 tiles)
-    const bool use_dmma = !fp32 && !zc && C.tune[PGPU_TUNE_DMMA] != 0 && !C.record;
+    const bool use_dmma = !fp32 && C.tune[PGPU_TUNE_DMMA] != 0 && !C.record;
     // tile shape of the tensor-core lists: tcgen05 tiles in single precision
     // (update tiles of LL^t / LU, and the TRSM tiles of every real form,
     // LDL^t included), DMMA tiles in FP64
@@ -1560,8 +1560,8 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem_bytes<true>()));
         PGPU_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, C.device));
     }
-    if constexpr (std::is_same<T, double>::value)
-        PGPU_CHECK(cudaFuncSetAttribute(k_gemm_scatter_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if constexpr (!F32)
+        PGPU_CHECK(cudaFuncSetAttribute(k_gemm_scatter_dmma<CPX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         dg_smem_bytes()));
     int64_t *prof[4] = {nullptr, nullptr, nullptr, nullptr};
     if (C.record) {
@@ -1628,11 +1628,12 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                 ngemm++;
             }
         }
-        if constexpr (std::is_same<T, double>::value) {
+        if constexpr (!F32) {
             if (ntc) {   // FP64 tensor cores (DMMA)
                 PGPU_CHECK(lt.mark(PH_TC));
-                k_gemm_scatter_dmma<<<ntc, DG_THREADS, dg_smem_bytes(), st>>>(
-                    C.meta, C.d_tctiles.p + c0, C.d_tasks.p, coefL, coefU, nullptr, nullptr, C.d_tmap.p, C.d_taux.p);
+                k_gemm_scatter_dmma<CPX><<<ntc, DG_THREADS, dg_smem_bytes(), st>>>(
+                    C.meta, C.d_tctiles.p + c0, C.d_tasks.p, reinterpret_cast<double *>(coefL),
+                    reinterpret_cast<double *>(coefU), nullptr, nullptr, C.d_tmap.p, C.d_taux.p);
                 if (la) PGPU_CHECK(lt.mark(PH_END));
                 nl++;
                 ngemm++;
@@ -1762,12 +1763,13 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                                                       inv, scr, nullptr);
                 nl++;
             }
-            if constexpr (std::is_same<T, double>::value) {
+            if constexpr (!F32) {
                 const int ntc = C.tttile_ptr[l + 1] - C.tttile_ptr[l];
                 if (ntc) {
-                    k_gemm_scatter_dmma<<<ntc, DG_THREADS, dg_smem_bytes(), s>>>(
-                        C.meta, C.d_tttiles.p + C.tttile_ptr[l], C.d_tasks.p, coefL, coefU, inv, scr, C.d_tmap.p,
-                        C.d_taux.p);
+                    k_gemm_scatter_dmma<CPX><<<ntc, DG_THREADS, dg_smem_bytes(), s>>>(
+                        C.meta, C.d_tttiles.p + C.tttile_ptr[l], C.d_tasks.p, reinterpret_cast<double *>(coefL),
+                        reinterpret_cast<double *>(coefU), reinterpret_cast<const double *>(inv),
+                        reinterpret_cast<double *>(scr), C.d_tmap.p, C.d_taux.p);
                     nl++;
                 }
             }

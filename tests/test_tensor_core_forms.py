@@ -52,7 +52,7 @@ def _error(A, st, fact, L, U):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("mixed", [True], ids=["mixed"])
+@pytest.mark.parametrize("mixed", [True, False], ids=["mixed", "fp64"])
 @pytest.mark.parametrize("fact,make", CASES, ids=IDS)
 def test_tensor_core_forms_match_restatement(fact, make, mixed):
     """Factors as close to the 64-bit restatement as the FMA tiles' (the tensor-core sums round less
