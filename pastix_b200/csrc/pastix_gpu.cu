@@ -1011,9 +1011,11 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                         for (int tn = 0; tn < cdiv((tc_trsm ? cs : 1) * w, bn); tn++)
                             (tc_trsm ? tttiles : ttiles).push_back(make_int4(id, tm, tn, 0));
                 }
-            } else if (h > fuse && h == w && tgemm) {
-                // a wide cblk without off-diagonal rows (a root): the inverse alone, for
-                // the solve's products with it (no TRSM)
+            } else if (tgemm && ((h > fuse && h == w) || (by_rows && rows_inv))) {
+                // a wide cblk without off-diagonal rows (a root), or whose rows the block-row
+                // kernel solved itself: the inverse alone, for the solve's products with it (no
+                // TRSM).  With it whole levels of short panels join the dataflow solve: 20^3 FP64
+                // solve 0.36 -> 0.26 ms, step of 128 2D systems 22.8 -> 20.9 ms
                 const int sides = lu ? 2 : 1;
                 C.invoff[c] = inv_elems;
                 inv_elems += sides * inv_span(w, C.ld[c]);
