@@ -152,6 +152,19 @@ template <typename R> __device__ __forceinline__ void atomic_sub(cplx<R> *p, con
     atomicAdd(&p->im, -v.im);
 }
 
+// a b + c with fused roundings.
+__device__ __forceinline__ float fma_v(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_v(double a, double b, double c) { return fma(a, b, c); }
+template <typename R> __device__ __forceinline__ cplx<R> fma_v(const cplx<R> &a, const cplx<R> &b, const cplx<R> &c) {
+    return cplx<R>(fma_v(-a.im, b.im, fma_v(a.re, b.re, c.re)), fma_v(a.im, b.re, fma_v(a.re, b.im, c.im)));
+}
+
+// Atomic add of 4 consecutive floats (16-byte aligned address).
+__device__ __forceinline__ void red_add_v4(float *p, float a, float b, float c, float d) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+
 // Task timing for the learned cost model: when prof != nullptr, thread 0 of
 // each CTA stores the global timer (ns) at the CTA's start and end in
 // prof[2 * blockIdx.x + {0, 1}].

@@ -410,13 +410,6 @@ constexpr int tcp_smem_bytes() {
 }
 constexpr int TCP_TMEM_COLS = 256;
 
-// Atomic add of 4 consecutive floats (16-byte aligned address).
-__device__ __forceinline__ void red_add_v4(float *p, float a, float b, float c, float d) {
-    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
-                 : "memory");
-}
-
-
 struct TcTileView {
     const float *A, *B;
     int mrows, ncols, K, nk, flags, c, b, f, arow, j0, i0, M, pair;

@@ -65,11 +65,6 @@ __host__ __device__ constexpr int pr_scr_tile(bool lu) { return (lu ? 2 : 1) * P
 // scratch tile of row 0}.
 enum { PR_ROW = 0, PR_INV = 1, PR_INV2 = 2 };
 
-__device__ __forceinline__ float fma_v(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fma_v(double a, double b, double c) { return fma(a, b, c); }
-template <typename R> __device__ __forceinline__ cplx<R> fma_v(const cplx<R> &a, const cplx<R> &b, const cplx<R> &c) {
-    return cplx<R>(fma_v(-a.im, b.im, fma_v(a.re, b.re, c.re)), fma_v(a.im, b.re, fma_v(a.re, b.im, c.im)));
-}
 template <typename T> __device__ __forceinline__ void ld16(const T *p, T (&v)[16 / sizeof(T)]) {
     const uint4 u = *reinterpret_cast<const uint4 *>(p);
     memcpy(v, &u, 16);
