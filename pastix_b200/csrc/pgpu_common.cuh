@@ -152,6 +152,17 @@ template <typename R> __device__ __forceinline__ void atomic_sub(cplx<R> *p, con
     atomicAdd(&p->im, -v.im);
 }
 
+// 16 bytes of consecutive elements (aligned addresses).
+template <typename T> __device__ __forceinline__ void ld16(const T *p, T (&v)[16 / sizeof(T)]) {
+    const uint4 u = *reinterpret_cast<const uint4 *>(p);
+    memcpy(v, &u, 16);
+}
+template <typename T> __device__ __forceinline__ void st16(T *p, const T (&v)[16 / sizeof(T)]) {
+    uint4 u;
+    memcpy(&u, v, 16);
+    *reinterpret_cast<uint4 *>(p) = u;
+}
+
 // a b + c with fused roundings.
 __device__ __forceinline__ float fma_v(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_v(double a, double b, double c) { return fma(a, b, c); }

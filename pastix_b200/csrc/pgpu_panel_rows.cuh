@@ -65,10 +65,6 @@ __host__ __device__ constexpr int pr_scr_tile(bool lu) { return (lu ? 2 : 1) * P
 // scratch tile of row 0}.
 enum { PR_ROW = 0, PR_INV = 1, PR_INV2 = 2 };
 
-template <typename T> __device__ __forceinline__ void ld16(const T *p, T (&v)[16 / sizeof(T)]) {
-    const uint4 u = *reinterpret_cast<const uint4 *>(p);
-    memcpy(v, &u, 16);
-}
 template <typename T> __device__ __forceinline__ void ldcg16(const T *p, T (&v)[16 / sizeof(T)]) {
     const uint4 u = __ldcg(reinterpret_cast<const uint4 *>(p));
     memcpy(v, &u, 16);
@@ -85,11 +81,6 @@ template <typename T> __device__ __forceinline__ T ldcg_s(const T *p) {   // one
     } else {
         return __ldcg(p);
     }
-}
-template <typename T> __device__ __forceinline__ void st16(T *p, const T (&v)[16 / sizeof(T)]) {
-    uint4 u;
-    memcpy(&u, v, 16);
-    *reinterpret_cast<uint4 *>(p) = u;
 }
 
 // acc[p][q] += sum_k A[a0 + p S][k] op(B[b0 + q S][k]) over one 32-column tile.
@@ -130,18 +121,29 @@ __device__ __forceinline__ bool pr_wait(const int *p, int need) {
     return true;
 }
 
+// Named barrier 1 + C: columns 8 C .. 8 C + 7 of the elimination are in shared memory (the eliminating
+// warp arrives, the inverse warps, one or two, wait).
+template <int C, int THREADS> __device__ __forceinline__ void pr_chunk_arrive() {
+    asm volatile("bar.arrive %0, %1;" ::"n"(C + 1), "n"(THREADS) : "memory");
+}
+template <int C, int THREADS> __device__ __forceinline__ void pr_chunk_sync() {
+    asm volatile("bar.sync %0, %1;" ::"n"(C + 1), "n"(THREADS) : "memory");
+}
+
 // Elimination of the nb x nb tile by one warp, lane = row, the row in
 // registers: a_ij -= l_ik d_k op(l_jk) (LU: l_ik u_kj) with l_ik = a_ik / d_k.
 // The active columns sit at a[0 ..]: each step shifts them down by one, so the
 // step loop needs no unrolling (its 32-fold body would miss in the instruction
 // cache) and the update no dynamic register index; after every 8 steps the
-// unrolled width shrinks by 8.  Column k of l goes to Lc[k][i - k - 1], row k
-// of u (LU) to Ub[k][j - k - 1], d_k and 1/d_k to dsm / rsm; *pk = k + 1 tells
-// the inverse warps that step k is there.  A negative Cholesky pivot becomes
-// NaN at once, as its square root would.
+// unrolled width shrinks by 8.  The next pivot needs only its own row's l, so
+// it goes to the other lanes (dn) before the column is exchanged: a step costs
+// a reciprocal, two products and a shuffle, the rest runs beside it.  Column k
+// of l goes to Lc[k][i - k - 1], row k of u (LU) to Ub[k][j - k - 1], d_k and
+// 1/d_k to dsm / rsm.  A negative Cholesky pivot becomes NaN at once, as its
+// square root would.
 template <typename T, int MODE, int W>
-__device__ __forceinline__ void pr_factor_steps(T (&a)[PB], int nb, typename real_of<T>::type crit, T *Lc, T *Ub,
-                                                T *dsm, T *rsm, volatile int *pk, int &npiv, int &nneg, int &nbad) {
+__device__ __forceinline__ void pr_factor_steps(T (&a)[PB], T &dn, int nb, typename real_of<T>::type crit, T *Lc,
+                                                T *Ub, T *dsm, T *rsm, int &npiv, int &nneg, int &nbad) {
     typedef typename real_of<T>::type R;
     constexpr bool LU = (MODE == FM_GETRF), CJ = fm_conj(MODE);
     constexpr int VK = pr_vk<T>();
@@ -149,7 +151,8 @@ __device__ __forceinline__ void pr_factor_steps(T (&a)[PB], int nb, typename rea
 #pragma unroll 1
     for (int k = PB - W; k < PB - W + 8; k++) {
         if (k >= nb) break;
-        T d = shfl_v(a[0], k);
+        T d = dn;
+        const T u1 = LU ? shfl_v(a[1], k) : T(0);
         if (!finite_v(d)) nbad++;
         d = static_pivot<T, MODE>(d, crit, npiv);
         if (CJ) d = T(real_v(d));   // (the diagonal of a Hermitian form is real)
@@ -161,6 +164,7 @@ __device__ __forceinline__ void pr_factor_steps(T (&a)[PB], int nb, typename rea
         const bool below = lane > k && lane < nb;
         const T raw = below ? a[0] : T(0);
         const T l = raw * r;
+        dn = shfl_v(LU ? fma_v(-l, u1, a[1]) : fma_v(-raw, cj<CJ>(l), a[1]), min(k + 1, 31));
         if (lane > k) Lc[k * PB + lane - k - 1] = l;
         if (lane == k) {
             dsm[k] = d;
@@ -174,9 +178,7 @@ __device__ __forceinline__ void pr_factor_steps(T (&a)[PB], int nb, typename rea
                     st16(Ub + k * PB + t, v);
                 }
         }
-        __threadfence_block();
         __syncwarp();
-        if (lane == 0) *pk = k + 1;
         const T x = LU ? l : raw;
         const T *col = (LU ? Ub : Lc) + k * PB;
 #pragma unroll
@@ -188,10 +190,11 @@ __device__ __forceinline__ void pr_factor_steps(T (&a)[PB], int nb, typename rea
                 if (t + q + 1 < W) a[t + q] = fma_v(-x, cj<CJ && !LU>(c[q]), a[t + q + 1]);
         }
     }
+    if (PB - W < nb) pr_chunk_arrive<(PB - W) / 8, LU ? 96 : 64>();
 }
 template <typename T, int MODE>
 __device__ __noinline__ void pr_factor_tile(const T *tile, int nb, typename real_of<T>::type crit, T *Lc, T *Ub,
-                                            T *dsm, T *rsm, volatile int *pk, Status *st) {
+                                            T *dsm, T *rsm, Status *st) {
     const int lane = threadIdx.x & 31;
     int npiv = 0, nneg = 0, nbad = 0;
     T a[PB];
@@ -202,11 +205,11 @@ __device__ __noinline__ void pr_factor_tile(const T *tile, int nb, typename real
 #pragma unroll
         for (int q = 0; q < pr_vk<T>(); q++) a[j + q] = (lane < nb && j + q < nb) ? v[q] : T(0);
     }
-    __syncwarp();
-    pr_factor_steps<T, MODE, 32>(a, nb, crit, Lc, Ub, dsm, rsm, pk, npiv, nneg, nbad);
-    pr_factor_steps<T, MODE, 24>(a, nb, crit, Lc, Ub, dsm, rsm, pk, npiv, nneg, nbad);
-    pr_factor_steps<T, MODE, 16>(a, nb, crit, Lc, Ub, dsm, rsm, pk, npiv, nneg, nbad);
-    pr_factor_steps<T, MODE, 8>(a, nb, crit, Lc, Ub, dsm, rsm, pk, npiv, nneg, nbad);
+    T dn = shfl_v(a[0], 0);
+    pr_factor_steps<T, MODE, 32>(a, dn, nb, crit, Lc, Ub, dsm, rsm, npiv, nneg, nbad);
+    pr_factor_steps<T, MODE, 24>(a, dn, nb, crit, Lc, Ub, dsm, rsm, npiv, nneg, nbad);
+    pr_factor_steps<T, MODE, 16>(a, dn, nb, crit, Lc, Ub, dsm, rsm, npiv, nneg, nbad);
+    pr_factor_steps<T, MODE, 8>(a, dn, nb, crit, Lc, Ub, dsm, rsm, npiv, nneg, nbad);
     if (lane == 0) {
         if (npiv) atomicAdd(&st->nbpivots, npiv);
         if (nneg) atomicAdd(&st->negpivots, nneg);
@@ -215,21 +218,15 @@ __device__ __noinline__ void pr_factor_tile(const T *tile, int nb, typename real
 }
 // Inverse of the unit lower factor whose columns are col[k][i - k - 1] (with
 // scale: of the lower factor with diagonal 1 / rsm[k], (U^t)^{-1}), one warp
-// behind the elimination, lane = column: out[k][lane].  Rows past nb of out
-// are the caller's zeros.
-template <typename T, int W>
-__device__ __forceinline__ bool pr_inverse_steps(T (&x)[PB], int nb, const T *col, const T *rsm, bool scale, T *out,
-                                                 volatile int *pk) {
+// eight columns behind the elimination, lane = column: out[k][lane].
+template <typename T, int THREADS, int W>
+__device__ __forceinline__ void pr_inverse_steps(T (&x)[PB], int nb, const T *col, const T *rsm, bool scale, T *out) {
     constexpr int VK = pr_vk<T>();
     const int lane = threadIdx.x & 31;
+    if (PB - W < nb) pr_chunk_sync<(PB - W) / 8, THREADS>();
 #pragma unroll 1
     for (int k = PB - W; k < PB - W + 8; k++) {
         if (k >= nb) break;
-        const long long t0 = clock64();
-        while (*pk <= k)
-            if (clock64() - t0 > PR_WAIT_CYCLES) return false;
-        __threadfence_block();
-        __syncwarp();
         T v = x[0];
         if (scale) v = v * rsm[k];
         out[k * pr_pitch<T>() + lane] = v;
@@ -243,19 +240,18 @@ __device__ __forceinline__ bool pr_inverse_steps(T (&x)[PB], int nb, const T *co
                 if (t + q + 1 < W) x[t + q] = fma_v(-cv[q], v, x[t + q + 1]);
         }
     }
-    return true;
 }
-template <typename T>
-__device__ __noinline__ bool pr_inverse_tile(int nb, const T *col, const T *rsm, bool scale, T *out,
-                                             volatile int *pk) {
+template <typename T, int THREADS>
+__device__ __noinline__ void pr_inverse_tile(int nb, const T *col, const T *rsm, bool scale, T *out) {
     const int lane = threadIdx.x & 31;
     T x[PB];
 #pragma unroll
     for (int i = 0; i < PB; i++) x[i] = T(i == lane ? 1 : 0);
-    return pr_inverse_steps<T, 32>(x, nb, col, rsm, scale, out, pk) &&
-           pr_inverse_steps<T, 24>(x, nb, col, rsm, scale, out, pk) &&
-           pr_inverse_steps<T, 16>(x, nb, col, rsm, scale, out, pk) &&
-           pr_inverse_steps<T, 8>(x, nb, col, rsm, scale, out, pk);
+    pr_inverse_steps<T, THREADS, 32>(x, nb, col, rsm, scale, out);
+    pr_inverse_steps<T, THREADS, 24>(x, nb, col, rsm, scale, out);
+    pr_inverse_steps<T, THREADS, 16>(x, nb, col, rsm, scale, out);
+    pr_inverse_steps<T, THREADS, 8>(x, nb, col, rsm, scale, out);
+    for (int k = nb; k < PB; k++) out[k * pr_pitch<T>() + lane] = T(0);   // (rows past a ragged tile)
 }
 
 template <typename T, int MODE>
@@ -270,12 +266,10 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
     extern __shared__ __align__(16) unsigned char pr_smem[];
     __shared__ __align__(16) T dsm[PB], rsm[PB], sqs[PB];
     __shared__ int job_s, fail_s;
-    __shared__ volatile int pk_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         job_s = atomicAdd(ticket, 1);
         fail_s = 0;
-        pk_s = 0;
     }
     __syncthreads();
     const int4 jb = jobs[job_s];
@@ -438,45 +432,40 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
         }
         __syncthreads();
         if (diag && !failed()) {
-            // the diagonal tile: elimination (warp 0), its inverse (warp 1; LU: U's on warp 2) a step behind
+            // the diagonal tile: elimination (warp 0), its inverse (warp 1; LU: U's on warp 2) behind it
             T *Lc = S, *To = S + TILE, *Ub = LU ? S + 2 * TILE : nullptr, *Vo = LU ? S + 3 * TILE : nullptr;
-            for (int e = tid; e < PB * P; e += PR_THREADS) {
-                To[e] = T(0);
-                if (LU) Vo[e] = T(0);
-            }
-            __syncthreads();
             const R crit = R(*critp);
-            if (warp == 0) {
-                pr_factor_tile<T, MODE>(row + i * TILE, nr, crit, Lc, Ub, dsm, rsm, &pk_s, st);
-            } else if (warp == 1 || (LU && warp == 2)) {
-                if (!pr_inverse_tile<T>(nr, warp == 1 ? Lc : Ub, rsm, warp == 2, warp == 1 ? To : Vo, &pk_s)) fail_s = 1;
-            }
+            if (warp == 0) pr_factor_tile<T, MODE>(row + i * TILE, nr, crit, Lc, Ub, dsm, rsm, st);
+            else if (warp == 1) pr_inverse_tile<T, LU ? 96 : 64>(nr, Lc, rsm, false, To);
+            else if (LU && warp == 2) pr_inverse_tile<T, 96>(nr, Ub, rsm, true, Vo);
             __syncthreads();
             if (MODE == FM_POTRF) {
                 if (tid < nr) sqs[tid] = sqrt_v(dsm[tid]);
                 __syncthreads();
             }
+            // what the other rows wait for first
             T *so = sc + (int64_t)i * SCR;
             for (int e = tid; e < PB * PB; e += PR_THREADS) {
                 const int r = e / PB, q = e % PB;
-                const bool in = r < nr && q < nr;
                 T t = To[r * P + q];
-                if (MODE == FM_POTRF && in) t = t * (T(1) / sqs[r]);
+                if (MODE == FM_POTRF && r < nr) t = t * (T(1) / sqs[r]);
                 so[e] = t;
                 if (LU) so[PB * PB + e] = Vo[r * P + q];
-                if (in && (LU || q <= r)) {
-                    T v;
-                    if (q == r) v = MODE == FM_POTRF ? sqs[r] : dsm[r];
-                    else if (q < r) v = MODE == FM_POTRF ? Lc[q * PB + r - q - 1] * sqs[q] : Lc[q * PB + r - q - 1];
-                    else v = Ub[r * PB + q - r - 1];
-                    A[(int64_t)(r0 + r) * ld + r0 + q] = v;
-                }
             }
             if (tid < PB) so[(LU ? 2 : 1) * PB * PB + tid] = tid < nr ? rsm[tid] : T(0);
             __syncthreads();
-            if (tid == 0 && !failed()) {
+            if (tid == 0) {
                 __threadfence();
                 atomicExch(pc + i, i + 1);
+            }
+            for (int e = tid; e < PB * PB; e += PR_THREADS) {
+                const int r = e / PB, q = e % PB;
+                if (r >= nr || q >= nr || (!LU && q > r)) continue;
+                T v;
+                if (q == r) v = MODE == FM_POTRF ? sqs[r] : dsm[r];
+                else if (q < r) v = MODE == FM_POTRF ? Lc[q * PB + r - q - 1] * sqs[q] : Lc[q * PB + r - q - 1];
+                else v = Ub[r * PB + q - r - 1];
+                A[(int64_t)(r0 + r) * ld + r0 + q] = v;
             }
         }
     } else {

@@ -8,9 +8,10 @@ import scipy.sparse as sp
 from oracle.restate import sopalin_np as NP
 from pastix_b200 import matrices as M
 
-# first cblk's width, rows below it: one and two tiles, ragged last tiles, a panel solved in the
+# first cblk's width, rows below it: the one-warp panels (at most 32 columns), one and two tiles, ragged last tiles, a panel solved in the
 # kernel (height at most 256) and one that goes through the inverse, the widest block accepted
-SHAPES = [(33, 1), (64, 40), (65, 31), (96, 33), (127, 200), (160, 129), (320, 64), (400, 7)]
+SHAPES = [(1, 5), (7, 40), (31, 33), (32, 64), (33, 1), (64, 40), (65, 31), (96, 33), (127, 200), (160, 129),
+          (320, 64), (400, 7)]
 FORMS = [("potrf", False), ("sytrf", False), ("getrf", False), ("potrf", True), ("hetrf", True), ("sytrf", True),
          ("getrf", True)]
 
@@ -88,12 +89,12 @@ def test_block_rows_match_restatement(fact, cplx, w, m, mixed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("col", [0, 37, 95])
-def test_negative_pivot_is_refused(col):
+@pytest.mark.parametrize("w,col", [(20, 0), (20, 19), (96, 0), (96, 37), (96, 95)])
+def test_negative_pivot_is_refused(w, col):
     """A negative pivot makes the Cholesky factor non-finite, as its square root would: the numfact fails."""
     from pastix_b200 import gpu as G
-    st = _structure(96, 30)
-    A = _matrix("potrf", False, 126, np.random.default_rng(3), neg=col)
+    st = _structure(w, 30)
+    A = _matrix("potrf", False, w + 30, np.random.default_rng(3), neg=col)
     s = _solver(A, st, "potrf", False)
     with pytest.raises(G.PastixGpuError):
         s.numfact(A.values)
