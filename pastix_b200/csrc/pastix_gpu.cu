@@ -203,7 +203,7 @@ struct pastix_gpu_s {
     // coeftab and of the inverses (3xTF32), one tensor map per (source cblk,
     // operand kind), split jobs {cblk, row, panel, -} per level
     bool tma = false;
-    bool forms_off = false;   // no room (or no tensor maps) for the LDL / complex planes
+    bool tma_failed = false, forms_off = false;   // no tensor maps; no room for the LDL / complex planes
     DArr<float> d_hilo, d_ihilo;
     // 3xFP16 operands (mixed GEMM mode 3): FP16 hi / lo planes [2][h16_plane]
     // of the source matrices, per-row inverse scales, and per operand map its
@@ -217,6 +217,7 @@ struct pastix_gpu_s {
     // the target rows of the tensor-core update tasks (k_task_rowmap)
     DArr<int64_t> d_taux;
     DArr<int> d_tmap, d_tlist;
+    DArr<TcSeg> d_tcseg;
     DArr<TcDesc> d_tcdesc, d_ttdesc;   // per tensor-core tile (update, TRSM): k_gemm_scatter_tc_tma's records
     // dataflow solve of runs of levels whose cblks all hold a diagonal-block
     // inverse (k_solve_flow): runs {first level, end level}, per run the task
@@ -459,7 +460,7 @@ extern "C" int pastix_gpu_structure(pastix_gpu_t *ctx, int64_t n, int64_t cblknb
     }
     PGPU_CHECK(C.d_solve_chunks.upload(sch, s));
     C.plan_fact = -1;
-    C.forms_off = false;
+    C.tma_failed = C.forms_off = false;
     C.fact_done = -1;
     C.d_coef.release();
     PGPU_CHECK(cudaStreamSynchronize(s));
@@ -584,6 +585,11 @@ static const int TRSM_TR = 32;   // panel rows per k_trsm_rows CTA
 // PGPU_TUNE_TRSM_GEMM (PASTIX_GPU_TRSM=rows disables the TRSM-as-GEMM path),
 // PGPU_TUNE_TRSM_GEMM_ROWS (256: panels taller than this take it),
 // PGPU_TUNE_TC_MIN_MN (8192: smallest M x N sent to the tensor cores).
+// Most sources summed in one tensor-core tile before it is scattered: 100^3 LL^t
+// factorization 50.2 / 47.2 / 44.4 / 44.4 ms at 1 / 2 / 4 / 8 sources, 80^3 LU
+// 34.9 / 32.5 / 31.9 / 31.8, 60^3 complex LDL^h 17.9 / 17.8 / 17.6 / 17.4 (more
+// only delays the updates: 16 took as long as 8).
+const int TC_FANIN = 8;
 enum { MG_FP32 = 0, MG_TF32 = 1, MG_3XTF32 = 2, MG_3XF16 = 3 };
 static void default_tuning(int64_t *t) {
     const char *e = getenv("PASTIX_GPU_MIXED_GEMM");
@@ -889,7 +895,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     // single precision: the large update and TRSM GEMMs on the tcgen05 tensor cores; the LDL and the
     // complex forms only as 3xFP16 with pre-split operands (D and the complex product live in the planes)
     const bool h16_forms = fp32 && mixed_gemm_mode(C) == MG_3XF16 && C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record &&
-                           C.tune[PGPU_TUNE_TC_TMA] != 0 && tensor_map_encoder() != nullptr && !C.forms_off;
+                           C.tune[PGPU_TUNE_TC_TMA] != 0 && tensor_map_encoder() != nullptr && !C.tma_failed && !C.forms_off;
     const bool use_tc = fp32 && tc_enabled(C) && ((!zc && (fmode == FM_POTRF || fmode == FM_GETRF)) || h16_forms);
     const int cs = zc ? 2 : 1;   // floats per element: the tensor-core tiles of complex tasks are real ones
     // FP64: the large update and TRSM GEMMs on the FP64 tensor cores (DMMA),
@@ -944,7 +950,44 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     C.ps_ptr.assign(C.nlevels + 1, 0);
     C.tile_crit.assign(C.nlevels, 0);
     C.tctile_crit.assign(C.nlevels, 0);
-    std::vector<int4> lt[2], ltc[2], lsm[2];   // this level's FMA (CTA / warp) and tensor-core tiles: [0] next-level targets, [1] others
+    std::vector<int4> lt[2], lsm[2];   // this level's FMA (CTA / warp) tiles: [0] next-level targets, [1] others
+    // tensor-core update tasks per level and part, each the lead of a batch (fan-in: below)
+    std::vector<std::vector<int>> tcl[2];
+    for (int k = 0; k < 2; k++) tcl[k].resize(C.nlevels);
+    std::vector<std::vector<int>> batches;   // tasks of each batch, the lead first
+    std::vector<int> batch_of;                // lead task -> batch, -1
+    // Fan-in (k_gemm_scatter_tc_tma): deferred tasks into the same rows and columns of a cblk, from
+    // the successive cblks of a separator chain, are summed in one tile and scattered once, in the
+    // level of the last of them.  Keyed by target cblk, columns, panel sides and the rows below.
+    const bool tma_mode = use_tc && (mixed_gemm_mode(C) == MG_3XTF32 || mixed_gemm_mode(C) == MG_3XF16) &&
+                          C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record && C.tune[PGPU_TUNE_TC_TMA] != 0 &&
+                          tensor_map_encoder() != nullptr && !C.tma_failed;
+    struct FanKey {
+        int f, r0, r1, flags, M;
+        uint64_t tail;
+        bool operator==(const FanKey &o) const {
+            return f == o.f && r0 == o.r0 && r1 == o.r1 && flags == o.flags && M == o.M && tail == o.tail;
+        }
+    };
+    struct FanHash {
+        size_t operator()(const FanKey &k) const {
+            uint64_t h = k.tail;
+            for (int v : {k.f, k.r0, k.r1, k.flags, k.M}) h = (h ^ (uint64_t)(uint32_t)v) * 0x9E3779B97F4A7C15ull;
+            return (size_t)(h ^ (h >> 29));
+        }
+    };
+    std::unordered_map<FanKey, std::vector<int>, FanHash> fan;
+    std::vector<uint64_t> row_tail;           // per block of the current cblk: hash of the blocks from it on
+    auto same_rows = [&](int ta, int tb) {    // the two tasks update the same rows (lists of blocks compared)
+        const GemmTask &x = tasks[ta], &y = tasks[tb];
+        auto first = [&](const GemmTask &g) { return g.arow0 == C.browoff[g.b] ? g.b : g.b + 1; };
+        int bx = first(x), by = first(y);
+        const int ex = C.fblok[x.c + 1], ey = C.fblok[y.c + 1];
+        if (ex - bx != ey - by) return false;
+        for (; bx < ex; bx++, by++)
+            if (C.bfrow[bx] != C.bfrow[by] || C.blrow[bx] != C.blrow[by]) return false;
+        return true;
+    };
     // warp tiles for narrow FMA updates (not while recording task timings:
     // those describe the CTA tiles)
     const bool small_ok = !C.record && esz <= 8;
@@ -953,10 +996,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
         int64_t scr_lvl = 0;
         int prscr = 0, pr_wmax = 0, nlvl = 0;
         for (int q = C.lvl_ptr[l]; q < C.lvl_ptr[l + 1]; q++) nlvl += C.width[C.lvl_cblks[q]] > PB;
-        for (int k = 0; k < 2; k++) {
-            lt[k].clear();
-            ltc[k].clear();
-        }
+        for (int k = 0; k < 2; k++) lt[k].clear();
         for (int q = C.lvl_ptr[l]; q < C.lvl_ptr[l + 1]; q++) {
             const int c = C.lvl_cblks[q];
             const int w = C.width[c], h = C.height[c];
@@ -1022,6 +1062,12 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 inverse_jobs(sides);
             }
             const int b1 = C.fblok[c + 1];
+            row_tail.assign(b1 - C.fblok[c] + 1, 0);
+            for (int b = b1 - 1; b > C.fblok[c]; b--) {
+                uint64_t x = row_tail[b + 1 - C.fblok[c]] * 0x9E3779B97F4A7C15ull + (uint64_t)C.bfrow[b];
+                x = (x ^ (x >> 31)) * 0xBF58476D1CE4E5B9ull + (uint64_t)C.blrow[b];
+                row_tail[b - C.fblok[c]] = x ^ (x >> 27);
+            }
             for (int b = C.fblok[c] + 1; b < b1; b++) {
                 const int f = C.bfcblk[b];
                 const int N = C.blrow[b] - C.bfrow[b] + 1;
@@ -1034,11 +1080,13 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                     gflops += fma_flops * M * N * w;
                     if ((use_tc || use_dmma) && tc_task(C, M, cs * N, cs * w)) {
                         tcflops += fma_flops * M * N * w;
-                        for (int tm = 0; tm < cdiv(M, tbm); tm++)
-                            for (int tn = 0; tn < cdiv(cs * N, tbn); tn++) {
-                                if ((flags & 8) && (int64_t)(tm + 1) * tbm <= (int64_t)tn * tbn / cs) continue;
-                                ltc[crit].push_back(make_int4(id, tm, tn, 0));
-                            }
+                        if (tma_mode && crit) {
+                            const int tail = (arow0 == C.browoff[b] ? b : b + 1) - C.fblok[c];
+                            fan[FanKey{f, C.bfrow[b], C.blrow[b], flags, M, row_tail[tail]}].push_back(id);
+                        } else {
+                            tcl[crit][l].push_back((int)batches.size());
+                            batches.push_back({id});
+                        }
                         return;
                     }
                     if (small_ok && N <= GS_TN) {   // narrow update: one warp per 32 rows
@@ -1066,13 +1114,8 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             lsm[k].clear();
         }
         C.tile_crit[l] = (int)lt[0].size();
-        C.tctile_crit[l] = (int)ltc[0].size();
-        for (int k = 0; k < 2; k++) {
-            tiles.insert(tiles.end(), lt[k].begin(), lt[k].end());
-            tctiles.insert(tctiles.end(), ltc[k].begin(), ltc[k].end());
-        }
+        for (int k = 0; k < 2; k++) tiles.insert(tiles.end(), lt[k].begin(), lt[k].end());
         C.tile_ptr[l + 1] = (int)tiles.size();
-        C.tctile_ptr[l + 1] = (int)tctiles.size();
         C.trsm_ptr[l + 1] = (int)trsm.size();
         C.pn_ptr[l + 1] = (int)pjobs.size();
         C.ps_ptr[l + 1] = (int)sjobs.size();
@@ -1087,11 +1130,50 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
         C.tttile_ptr[l + 1] = (int)tttiles.size();
         scr_max = std::max(scr_max, scr_lvl);
     }
+    // the deferred tasks' batches: runs of at most TC_FANIN sources of a key in level order, the first
+    // one shorter by a phase that differs between targets (or every target of a chain would fall due
+    // in the same level); a batch runs in the level of its last source
+    {
+        std::vector<std::vector<int> *> groups;
+        for (auto &kv : fan) groups.push_back(&kv.second);
+        std::sort(groups.begin(), groups.end(),
+                  [](const std::vector<int> *x, const std::vector<int> *y) { return x->front() < y->front(); });
+        for (const std::vector<int> *g : groups) {
+            const int phase = tasks[g->front()].f % TC_FANIN;
+            size_t i = 0, lim = 1 + phase;
+            while (i < g->size()) {
+                std::vector<int> bt;
+                while (i < g->size() && bt.size() < lim && (bt.empty() || same_rows(bt[0], (*g)[i]))) bt.push_back((*g)[i++]);
+                lim = TC_FANIN;
+                tcl[1][C.cblk_level[tasks[bt.back()].c]].push_back((int)batches.size());
+                batches.push_back(std::move(bt));
+            }
+        }
+    }
+    batch_of.assign(tasks.size(), -1);
+    for (size_t i = 0; i < batches.size(); i++) batch_of[batches[i][0]] = (int)i;
+    // their tiles, the deepest sums first (the persistent kernel deals them out in this order)
+    for (int l = 0; l < C.nlevels; l++) {
+        for (int k = 0; k < 2; k++) {
+            std::stable_sort(tcl[k][l].begin(), tcl[k][l].end(),
+                             [&](int x, int y) { return batches[x].size() > batches[y].size(); });
+            for (int bi : tcl[k][l]) {
+                const int id = batches[bi][0];
+                const GemmTask &g = tasks[id];
+                const int N = C.blrow[g.b] - C.bfrow[g.b] + 1;
+                for (int tm = 0; tm < cdiv(g.M, tbm); tm++)
+                    for (int tn = 0; tn < cdiv(cs * N, tbn); tn++) {
+                        if ((g.flags & 8) && (int64_t)(tm + 1) * tbm <= (int64_t)tn * tbn / cs) continue;
+                        tctiles.push_back(make_int4(id, tm, tn, 0));
+                    }
+            }
+            if (k == 0) C.tctile_crit[l] = (int)tctiles.size() - C.tctile_ptr[l];
+        }
+        C.tctile_ptr[l + 1] = (int)tctiles.size();
+    }
     // TMA operands (3xTF32, persistent kernel): hi/lo mirrors, tensor maps of
     // the source cblks, split jobs of their off-diagonal rows per level
-    C.tma = use_tc && (mixed_gemm_mode(C) == MG_3XTF32 || mixed_gemm_mode(C) == MG_3XF16) &&
-            C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record &&
-            C.tune[PGPU_TUNE_TC_TMA] != 0 && tensor_map_encoder() != nullptr;
+    C.tma = tma_mode;
     C.split_ptr.assign(C.nlevels + 1, 0);
     C.h16 = C.tma && mixed_gemm_mode(C) == MG_3XF16;
     std::vector<int> mapidx_h;        // operand maps of each source cblk (TMA modes), for the tile descriptors
@@ -1100,7 +1182,8 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
         // 3xFP16: FP16 planes and row scales of the source matrices only (the
         // panels and inverses that feed a tensor-core task), in level order
         std::vector<char> src(C.cblknbr, 0);
-        for (const int4 &t : tctiles) src[tasks[t.x].c] = 1;
+        for (const auto &bt : batches)
+            for (int id : bt) src[tasks[id].c] = 1;
         for (const int4 &t : tttiles) src[tasks[t.x].c] = 1;
         std::vector<int> mapidx(C.cblknbr, -1);
         std::vector<int64_t> hoff, hsbase;
@@ -1186,16 +1269,13 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             mapidx_h.swap(mapidx);
             hsbase_h.swap(hsbase);
         } else {
-            if (zc || ldl) {   // (their tiles have no other tensor-core kernel)
-                C.forms_off = true;
-                return build_fact_plan(C, fmode, fp32, zc);
-            }
-            C.h16 = false;
-            C.split_ptr.assign(C.nlevels + 1, 0);
+            C.tma_failed = true;   // (a map the encoder refuses: plan without TMA)
+            return build_fact_plan(C, fmode, fp32, zc);
         }
     } else if (C.tma) {
         std::vector<char> src(C.cblknbr, 0);
-        for (const int4 &t : tctiles) src[tasks[t.x].c] = 1;
+        for (const auto &bt : batches)
+            for (int id : bt) src[tasks[id].c] = 1;
         for (const int4 &t : tttiles) src[tasks[t.x].c] = 1;
         const int64_t ncoef = C.coefnbr * (lu ? 2 : 1);
         C.hilo_plane = (ncoef + 31) / 32 * 32;
@@ -1238,7 +1318,8 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             mapidx_h = mapidx;
             PGPU_CHECK(C.d_split.upload(split, C.stream));
         } else {
-            C.split_ptr.assign(C.nlevels + 1, 0);
+            C.tma_failed = true;
+            return build_fact_plan(C, fmode, fp32, zc);
         }
     }
     if (C.tma) {
@@ -1345,6 +1426,39 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
         }
         PGPU_CHECK(C.d_taux.upload(taux, s));
         if (C.tma) {
+            // one segment per task, a batch's contiguous
+            std::vector<TcSeg> segs;
+            std::vector<int> seg0(tasks.size(), -1);
+            auto add_seg = [&](int id) {
+                const GemmTask &g = tasks[id];
+                const bool trsm = (g.flags & 64) != 0;
+                const int ka = ((g.flags & 1) || (ldl && !trsm)) ? TMAP_U : TMAP_L;
+                const int kb = trsm ? ((g.flags & 128) ? TMAP_I2 : TMAP_I)
+                                    : ((g.flags & 2) ? (zc ? TMAP_BU : TMAP_U) : (zc ? TMAP_BL : TMAP_L));
+                const int mb = mapidx_h[g.c];
+                TcSeg e;
+                std::memset(&e, 0, sizeof(e));
+                e.mapa = mb + ka;
+                e.mapb = mb + kb;
+                e.rowa = g.arow0;
+                e.rowb = cs * (trsm ? 0 : C.browoff[g.b]);
+                e.nk = cdiv(cs * C.width[g.c], C.h16 ? 64 : TC_BK);
+                if (C.h16) {
+                    e.sa = hsbase_h[mb + ka] + e.rowa;
+                    e.sb = hsbase_h[mb + kb] + e.rowb;
+                }
+                segs.push_back(e);
+            };
+            for (const auto &bt : batches) {
+                seg0[bt[0]] = (int)segs.size();
+                for (int id : bt) add_seg(id);
+            }
+            for (const int4 &t : tttiles)
+                if (seg0[t.x] < 0) {
+                    seg0[t.x] = (int)segs.size();
+                    add_seg(t.x);
+                }
+            PGPU_CHECK(C.d_tcseg.upload(segs, s));
             // one descriptor per tensor-core tile (k_gemm_scatter_tc_tma reads no task tables)
             auto make_desc = [&](const int4 &t) {
                 const GemmTask &g = tasks[t.x];
@@ -1352,21 +1466,16 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 const int c = g.c, w = C.width[c];
                 const int N = cs * (trsm ? w : C.blrow[g.b] - C.bfrow[g.b] + 1);
                 const int i0 = t.y * TC_BM, j0 = t.z * TC_BN;
-                const int ka = ((g.flags & 1) || (ldl && !trsm)) ? TMAP_U : TMAP_L;
-                const int kb = trsm ? ((g.flags & 128) ? TMAP_I2 : TMAP_I)
-                                    : ((g.flags & 2) ? (zc ? TMAP_BU : TMAP_U) : (zc ? TMAP_BL : TMAP_L));
-                const int mb = mapidx_h[c];
                 TcDesc d;
                 std::memset(&d, 0, sizeof(d));
-                d.mapa = mb + ka;
-                d.mapb = mb + kb;
-                d.rowa = g.arow0 + i0;
-                d.rowb = cs * (trsm ? 0 : C.browoff[g.b]) + j0;
-                d.nk = cdiv(cs * w, C.h16 ? 64 : TC_BK);
+                d.seg0 = seg0[t.x];
+                d.nseg = trsm ? 1 : (int)batches[batch_of[t.x]].size();
                 d.ncols = std::min(TC_BN, N - j0);
                 d.pair = t.w & 1;
                 d.flags = g.flags | (zc ? TC_FLAG_CPLX : 0);
                 d.mrows = g.M - i0;
+                d.i0 = i0;
+                d.j0 = j0;
                 if (trsm) {
                     d.ldo = cs * C.ld[c];
                     d.off = cs * (g.out + (int64_t)i0 * C.ld[c]) + j0;
@@ -1377,10 +1486,6 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                     d.tcol = cs * (C.bfrow[g.b] - C.fcol[f]) + j0;
                     d.off = cs * (((g.flags & 4) ? C.coefnbr : 0) + C.coefoff[f]);
                     d.rmap = taux[t.x] + i0;
-                }
-                if (C.h16) {
-                    d.sa = hsbase_h[mb + ka] + d.rowa;
-                    d.sb = hsbase_h[mb + kb] + d.rowb;
                 }
                 return d;
             };
@@ -1645,7 +1750,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
             if (ntc) {   // (planned for the 3xFP16 operands only)
                 PGPU_CHECK(lt.mark(PH_TC));
                 k_gemm_scatter_tc_tma<true, true><<<std::min(ntc, gcap), TMA_THREADS, tma_smem_bytes<true>(), st>>>(
-                    C.d_tcdesc.p + c0, ntc, reinterpret_cast<float *>(coefL), C.d_status.p, nullptr, C.d_tmaps.p,
+                    C.d_tcdesc.p + c0, C.d_tcseg.p, ntc, reinterpret_cast<float *>(coefL), C.d_status.p, nullptr, C.d_tmaps.p,
                     C.d_tmap.p, C.d_hscale.p);
                 if (la) PGPU_CHECK(lt.mark(PH_END));
                 nl++;
@@ -1658,12 +1763,12 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                 if (persist && C.tma && C.h16) {
                     const int g = std::min(ntc, gcap);
                     k_gemm_scatter_tc_tma<true, true><<<g, TMA_THREADS, tma_smem_bytes<true>(), st>>>(
-                        C.d_tcdesc.p + c0, ntc, coefL, C.d_status.p, nullptr, C.d_tmaps.p, C.d_tmap.p,
+                        C.d_tcdesc.p + c0, C.d_tcseg.p, ntc, coefL, C.d_status.p, nullptr, C.d_tmaps.p, C.d_tmap.p,
                         C.d_hscale.p);
                 } else if (persist && C.tma) {
                     const int g = std::min(ntc, gcap);
                     k_gemm_scatter_tc_tma<true><<<g, TMA_THREADS, tma_smem_bytes<true>(), st>>>(
-                        C.d_tcdesc.p + c0, ntc, coefL, C.d_status.p, nullptr, C.d_tmaps.p, C.d_tmap.p);
+                        C.d_tcdesc.p + c0, C.d_tcseg.p, ntc, coefL, C.d_status.p, nullptr, C.d_tmaps.p, C.d_tmap.p);
                 } else if (persist) {
                     const int g = std::min(ntc, gcap);
                     if (split)
@@ -1779,7 +1884,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                 const int ntc = C.tttile_ptr[l + 1] - C.tttile_ptr[l];
                 if (ntc) {
                     k_gemm_scatter_tc_tma<true, true><<<std::min(ntc, nsm), TMA_THREADS, tma_smem_bytes<true>(), s>>>(
-                        C.d_ttdesc.p + C.tttile_ptr[l], ntc, reinterpret_cast<float *>(coefL), C.d_status.p,
+                        C.d_ttdesc.p + C.tttile_ptr[l], C.d_tcseg.p, ntc, reinterpret_cast<float *>(coefL), C.d_status.p,
                         reinterpret_cast<float *>(scr), C.d_tmaps.p, C.d_tmap.p, C.d_hscale.p);
                     nl++;
                 }
@@ -1790,11 +1895,11 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                     const int g = std::min(ntc, nsm);
                     if (C.tma && C.h16)
                         k_gemm_scatter_tc_tma<true, true><<<g, TMA_THREADS, tma_smem_bytes<true>(), s>>>(
-                            C.d_ttdesc.p + C.tttile_ptr[l], ntc, coefL, C.d_status.p, scr, C.d_tmaps.p, C.d_tmap.p,
+                            C.d_ttdesc.p + C.tttile_ptr[l], C.d_tcseg.p, ntc, coefL, C.d_status.p, scr, C.d_tmaps.p, C.d_tmap.p,
                             C.d_hscale.p);
                     else if (C.tma)
                         k_gemm_scatter_tc_tma<true><<<g, TMA_THREADS, tma_smem_bytes<true>(), s>>>(
-                            C.d_ttdesc.p + C.tttile_ptr[l], ntc, coefL, C.d_status.p, scr, C.d_tmaps.p, C.d_tmap.p);
+                            C.d_ttdesc.p + C.tttile_ptr[l], C.d_tcseg.p, ntc, coefL, C.d_status.p, scr, C.d_tmaps.p, C.d_tmap.p);
                     else if (split)
                         k_gemm_scatter_tc_persistent<true><<<g, TCP_THREADS, tcp_smem_bytes<true>(), s>>>(
                             C.meta, C.d_tttiles.p + C.tttile_ptr[l], ntc, C.d_tasks.p, coefL, coefU, C.d_status.p,

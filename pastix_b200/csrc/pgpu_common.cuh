@@ -242,6 +242,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
         if (clock64() - t0 > 4000000000LL) return false;
     }
 }
+// The same by a whole warp, which goes on converged (its lanes leave the spin one by one).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(addr, parity));
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t addr) {
     asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(addr) : "memory");
 }

@@ -14,14 +14,14 @@
 // cover the coeftab itself, {K, rows, 1}.  Rows and columns past the panel
 // are zero-filled by the TMA unit.
 //
-// Roles (320 threads, one CTA per SM walking the level's tiles):
-//   warps 0-3, 6-9: epilogue (TMEM -> registers -> a swizzled 32 x 32 shared
-//              buffer per warp -> 16-byte vector reductions along the target
-//              rows);
-//   warp 4, lane 0: TMA producer -- per k-block waits for a free stage,
+// Roles (384 threads, one CTA per SM walking the level's tiles):
+//   warps 0-7: epilogue (TMEM -> registers, summed over the tile's segments
+//              -> a swizzled 32 x 32 shared buffer per warp -> 16-byte vector
+//              reductions along the target rows);
+//   warp 8, lane 0: TMA producer -- per k-block waits for a free stage,
 //              announces the stage's bytes on its mbarrier and issues the A
 //              and B box loads;
-//   warp 5, lane 0: MMA issuer (tcgen05.mma into one of two TMEM
+//   warp 9, lane 0: MMA issuer (tcgen05.mma into one of two TMEM
 //              accumulators, commits to the stage / accumulator barriers).
 // Every wait is bounded; after a time-out the producer waits (bounded) for
 // the loads it issued and TMEM is freed after all roles met.  The tensor
@@ -38,11 +38,15 @@
 
 namespace pgpu {
 
-// warps 0-3 and 6-9 write back the accumulators (two warps per TMEM lane
-// quarter, each taking every other 32-column chunk), warp 4 loads, warp 5
-// issues the MMAs
-constexpr int TMA_THREADS = 320, TMA_EPI_WARPS = 8;
-constexpr int TMA_PROD_WARP = 4, TMA_MMA_WARP = 5;
+// warps 0-7 gather and write back the accumulators (two warps per TMEM lane
+// quarter, each taking every other 32-column chunk), warp 8 loads, warp 9
+// issues the MMAs.  The epilogue warps hold a pair's sums (128 registers), so
+// the third warpgroup hands them registers: 2 x 208 + 88 = 3 x 168, the
+// launch's own share of 384 threads.
+constexpr int TMA_THREADS = 384, TMA_EPI_WARPS = 8;
+constexpr int TMA_PROD_WARP = 8, TMA_MMA_WARP = 9;
+constexpr int TMA_REGS_EPI = 208, TMA_REGS_REST = 88;
+static_assert(2 * TMA_REGS_EPI + TMA_REGS_REST == 3 * 168, "register split");
 constexpr int TMA_EPI_BYTES = TMA_EPI_WARPS * 32 * 32 * 4;   // a swizzled 32 x 32 float buffer per warp
 // operand maps per cblk: L panel, U panel (LU; LDL: the L rows times D), first / second diagonal-block
 // inverse, and in complex arithmetic the L / U panels as B operands (two real rows per row, see below)
@@ -72,27 +76,42 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
 }
 
 // Everything the three roles need for one tile, built on the host when the
-// plan is made: the kernel reads one 96-byte record per tile (loaded one or
-// two tiles ahead) instead of walking tile -> task -> cblk tables through
-// chains of dependent loads before it can issue a tile's loads or MMAs.
+// plan is made: the kernel reads one 64-byte record per tile and one 48-byte
+// record per segment (loaded one or two ahead) instead of walking tile -> task
+// -> cblk tables through chains of dependent loads.
+//
+// A tile sums nseg segments: update tasks of different source cblks with the
+// same target rows and columns (the cblks of one separator chain), each a
+// product of its own depth and row scales.  The epilogue warps gather the
+// segments' accumulators in registers and scatter the sum once: the atomic
+// reductions into the target panel, which bound the kernel when every source
+// writes its own (100^3: 41 GB of them), shrink by the number of segments.  A
+// tile of one segment goes chunk by chunk from the accumulator to the target
+// (through the registers of a whole tile it took a third longer).  With the
+// fan-in what bounds the kernel is the latency of its loads: on 72^3, tensor
+// pipe 43 % of active cycles, L2 23 %, DRAM below 15 %.
+struct __align__(16) TcSeg {
+    int mapa, mapb, rowa, rowb;   // tensor maps (indices into maps), first row of the task in A and in B
+    int nk, pad[3];               // k-blocks
+    int64_t sa, sb;               // 3xFP16: scale index of those rows
+};
 struct __align__(16) TcDesc {
-    int mapa, mapb, rowa, rowb;   // tensor maps (indices into maps) and row coordinates of A and B
-    int nk, ncols, pair, flags;   // k-blocks, valid columns, paired 128-row tiles, task flags (64: TRSM)
-    int mrows, ldo, wf, tcol;     // rows from the tile's first; target (or output) row stride, target
-                                  // cblk width (lower-triangle rule), first target column
-    int pad[4];
+    int seg0, nseg, ncols, pair;  // segments, valid columns, paired 128-row tiles
+    int flags, mrows, ldo, wf;    // task flags (64: TRSM), rows from the tile's first; target (or output) row
+                                  // stride, target cblk width (lower-triangle rule)
+    int tcol, i0, j0, pad;        // first target column; the tile's first row and column in its task
     int64_t off;                  // target panel offset from coefL, or (TRSM) output offset in scr
     int64_t rmap;                 // row-map index of the tile's first row (update tiles)
-    int64_t sa, sb;               // 3xFP16: scale index of the first A row, of the first B row
 };
-static_assert(sizeof(TcDesc) == 96, "TcDesc is six 16-byte vectors");
+static_assert(sizeof(TcSeg) == 48 && sizeof(TcDesc) == 64, "whole 16-byte vectors");
 
-__device__ __forceinline__ TcDesc tc_desc_load(const TcDesc *p) {
-    TcDesc d;
+template <typename R>
+__device__ __forceinline__ R tc_rec_load(const R *p) {
+    R d;
     const int4 *s = reinterpret_cast<const int4 *>(p);
     int4 *o = reinterpret_cast<int4 *>(&d);
 #pragma unroll
-    for (int k = 0; k < 6; k++) o[k] = __ldg(s + k);
+    for (int k = 0; k < (int)(sizeof(R) / 16); k++) o[k] = __ldg(s + k);
     return d;
 }
 
@@ -112,13 +131,11 @@ __device__ __forceinline__ TcDesc tc_desc_load(const TcDesc *p) {
 // of B becomes two, whose products with it are the real and the imaginary
 // part -- (re, -im) and (im, re), or for op = conj (re, im) and (-im, re) --
 // so that neighbouring columns of the accumulator are re and im, as in the
-// target panel, and the epilogue is the real one.  The planes of a complex
-// panel are three times its size, written once per cblk.  Measured on one
-// B200 against the FMA tiles: 60^3 complex64 LDL^h factorization 59.4 -> 18.7
-// ms, 53x49x61 real LDL^t 9.9 -> 5.7 ms.
+// target panel, and the epilogue is the real one.
 template <bool SPLIT, bool F16 = false>
 __global__ void __launch_bounds__(TMA_THREADS, 1)
-    k_gemm_scatter_tc_tma(const TcDesc *__restrict__ desc, int ntiles, float *__restrict__ coefL, Status *st,
+    k_gemm_scatter_tc_tma(const TcDesc *__restrict__ desc, const TcSeg *__restrict__ segs, int ntiles,
+                          float *__restrict__ coefL, Status *st,
                           float *__restrict__ scr, const CUtensorMap *__restrict__ maps,
                           const int *__restrict__ tmap, const float *__restrict__ hscale = nullptr) {
     static_assert(!F16 || SPLIT, "the FP16 operands are always split");
@@ -163,34 +180,43 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
     auto tile_addr = [&](int s, int q) { return base + (uint32_t)(s * NT + q) * TC_TILE_BYTES; };
     auto failed = [&]() { return *(volatile int *)&fail_s != 0; };
 
+    if (warp >= TMA_EPI_WARPS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TMA_REGS_REST));
     if (warp == TMA_PROD_WARP) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             int it = 0;
             TcDesc nx{};
-            if (blockIdx.x < ntiles) nx = tc_desc_load(desc + blockIdx.x);
-            for (int ti = blockIdx.x; ti < ntiles && !failed(); ti += gridDim.x) {
+            TcSeg ns{};
+            if (blockIdx.x < ntiles) {
+                nx = tc_rec_load(desc + blockIdx.x);
+                ns = tc_rec_load(segs + nx.seg0);
+            }
+            bool ok = true;
+            for (int ti = blockIdx.x; ti < ntiles && ok && !failed(); ti += gridDim.x) {
                 const TcDesc o = nx;
-                if (ti + (int)gridDim.x < ntiles) nx = tc_desc_load(desc + ti + gridDim.x);   // for the next tile
-                const CUtensorMap *ma = maps + o.mapa, *mbm = maps + o.mapb;
-                const int rowa = o.rowa, rowb = o.rowb, nk = o.nk;
+                const bool more = ti + (int)gridDim.x < ntiles;
+                if (more) nx = tc_rec_load(desc + ti + gridDim.x);   // for the next tile
                 const uint32_t bytes = (o.pair ? 3u : 2u) * BOX_BYTES;
-                bool ok = true;
-                for (int kb = 0; kb < nk; kb++, it++) {
-                    const int s = it % S;
-                    if (it >= S && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((it / S - 1) & 1))) {
-                        ok = false;
-                        break;
+                for (int g = 0; g < o.nseg && ok; g++) {
+                    const TcSeg sg = ns;
+                    if (g + 1 < o.nseg) ns = tc_rec_load(segs + o.seg0 + g + 1);
+                    else if (more) ns = tc_rec_load(segs + nx.seg0);
+                    const CUtensorMap *ma = maps + sg.mapa, *mbm = maps + sg.mapb;
+                    const int rowa = sg.rowa + o.i0, rowb = sg.rowb + o.j0;
+                    for (int kb = 0; kb < sg.nk; kb++, it++) {
+                        const int s = it % S;
+                        if (it >= S && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((it / S - 1) & 1))) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_arrive_expect_tx(smem_u32(&full[s]), bytes);
+                        tma_load_3d(tile_addr(s, 0), ma, kb * BK, rowa, 0, smem_u32(&full[s]));
+                        if (o.pair) tma_load_3d(tile_addr(s, QA1), ma, kb * BK, rowa + TC_BM, 0, smem_u32(&full[s]));
+                        tma_load_3d(tile_addr(s, QB), mbm, kb * BK, rowb, 0, smem_u32(&full[s]));
                     }
-                    mbar_arrive_expect_tx(smem_u32(&full[s]), bytes);
-                    tma_load_3d(tile_addr(s, 0), ma, kb * BK, rowa, 0, smem_u32(&full[s]));
-                    if (o.pair) tma_load_3d(tile_addr(s, QA1), ma, kb * BK, rowa + TC_BM, 0, smem_u32(&full[s]));
-                    tma_load_3d(tile_addr(s, QB), mbm, kb * BK, rowb, 0, smem_u32(&full[s]));
                 }
-                if (!ok) {
-                    atomicExch(&fail_s, 1);
-                    break;
-                }
+                if (!ok) atomicExch(&fail_s, 1);
             }
             if (failed()) {
                 // the loads still in flight land before the CTA leaves; if one
@@ -206,153 +232,141 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
     } else if (warp == TMA_MMA_WARP) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            int it = 0, tl = 0;
+            int it = 0, cnt = 0;   // k-blocks, segments
             TcDesc nx{};
-            if (blockIdx.x < ntiles) nx = tc_desc_load(desc + blockIdx.x);
-            for (int ti = blockIdx.x; ti < ntiles && !failed(); ti += gridDim.x, tl++) {
+            TcSeg ns{};
+            if (blockIdx.x < ntiles) {
+                nx = tc_rec_load(desc + blockIdx.x);
+                ns = tc_rec_load(segs + nx.seg0);
+            }
+            bool ok = true;
+            for (int ti = blockIdx.x; ti < ntiles && ok && !failed(); ti += gridDim.x) {
                 const TcDesc v = nx;
-                if (ti + (int)gridDim.x < ntiles) nx = tc_desc_load(desc + ti + gridDim.x);   // for the next tile
+                const bool more = ti + (int)gridDim.x < ntiles;
+                if (more) nx = tc_rec_load(desc + ti + gridDim.x);   // for the next tile
                 const uint32_t idesc = F16 ? tc_idesc_f16(tc_mma_n(v.ncols)) : tc_idesc(tc_mma_n(v.ncols));
-                const int vnk = v.nk;
-                const int ab = tl & 1;
-                const uint32_t acc = tmem + (uint32_t)(ab * 256), acc1 = acc + 128u;
                 const bool pair = v.pair != 0;
-                if (tl >= 2 && !mbar_wait(smem_u32(&acce[ab]), (uint32_t)((tl / 2 - 1) & 1))) {
-                    atomicExch(&fail_s, 1);
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                bool ok = true;
-                for (int kb = 0; kb < vnk; kb++, it++) {
-                    const int s = it % S;
-                    if (!mbar_wait(smem_u32(&full[s]), (uint32_t)((it / S) & 1))) {
+                for (int g = 0; g < v.nseg && ok; g++, cnt++) {
+                    const TcSeg sg = ns;
+                    if (g + 1 < v.nseg) ns = tc_rec_load(segs + v.seg0 + g + 1);
+                    else if (more) ns = tc_rec_load(segs + nx.seg0);
+                    const int ab = cnt & 1;
+                    const uint32_t acc = tmem + (uint32_t)(ab * 256), acc1 = acc + 128u;
+                    if (cnt >= 2 && !mbar_wait(smem_u32(&acce[ab]), (uint32_t)((cnt / 2 - 1) & 1))) {
                         ok = false;
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                    for (int kk = 0; kk < TC_BK / 8; kk++) {
-                        const uint32_t first = (kb > 0 || kk > 0) ? 1u : 0u;
-                        if (SPLIT) {
-                            const uint64_t bh = tc_sdesc(tile_addr(s, QB) + kk * 32),
-                                           bl = tc_sdesc(tile_addr(s, QB + 1) + kk * 32);
-#pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                if (h == 1 && !pair) break;
-                                const uint64_t ah = tc_sdesc(tile_addr(s, h * QA1) + kk * 32),
-                                               al = tc_sdesc(tile_addr(s, h * QA1 + 1) + kk * 32);
-                                const uint32_t ac = h ? acc1 : acc;
-                                if (F16) {
-                                    tc_mma_f16(ac, al, bh, idesc, first);
-                                    tc_mma_f16(ac, ah, bl, idesc, 1u);
-                                    tc_mma_f16(ac, ah, bh, idesc, 1u);
-                                } else {
-                                    tc_mma(ac, al, bh, idesc, first);
-                                    tc_mma(ac, ah, bl, idesc, 1u);
-                                    tc_mma(ac, ah, bh, idesc, 1u);
-                                }
-                            }
-                        } else {
-                            const uint64_t bd = tc_sdesc(tile_addr(s, QB) + kk * 32);
-                            tc_mma(acc, tc_sdesc(tile_addr(s, 0) + kk * 32), bd, idesc, first);
-                            if (pair) tc_mma(acc1, tc_sdesc(tile_addr(s, QA1) + kk * 32), bd, idesc, first);
+                    for (int kb = 0; kb < sg.nk; kb++, it++) {
+                        const int s = it % S;
+                        if (!mbar_wait(smem_u32(&full[s]), (uint32_t)((it / S) & 1))) {
+                            ok = false;
+                            break;
                         }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    #pragma unroll
+                        for (int kk = 0; kk < TC_BK / 8; kk++) {
+                            const uint32_t first = (kb > 0 || kk > 0) ? 1u : 0u;
+                            if (SPLIT) {
+                                const uint64_t bh = tc_sdesc(tile_addr(s, QB) + kk * 32),
+                                               bl = tc_sdesc(tile_addr(s, QB + 1) + kk * 32);
+    #pragma unroll
+                                for (int h = 0; h < 2; h++) {
+                                    if (h == 1 && !pair) break;
+                                    const uint64_t ah = tc_sdesc(tile_addr(s, h * QA1) + kk * 32),
+                                                   al = tc_sdesc(tile_addr(s, h * QA1 + 1) + kk * 32);
+                                    const uint32_t ac = h ? acc1 : acc;
+                                    if (F16) {
+                                        tc_mma_f16(ac, al, bh, idesc, first);
+                                        tc_mma_f16(ac, ah, bl, idesc, 1u);
+                                        tc_mma_f16(ac, ah, bh, idesc, 1u);
+                                    } else {
+                                        tc_mma(ac, al, bh, idesc, first);
+                                        tc_mma(ac, ah, bl, idesc, 1u);
+                                        tc_mma(ac, ah, bh, idesc, 1u);
+                                    }
+                                }
+                            } else {
+                                const uint64_t bd = tc_sdesc(tile_addr(s, QB) + kk * 32);
+                                tc_mma(acc, tc_sdesc(tile_addr(s, 0) + kk * 32), bd, idesc, first);
+                                if (pair) tc_mma(acc1, tc_sdesc(tile_addr(s, QA1) + kk * 32), bd, idesc, first);
+                            }
+                        }
+                        tc_commit(smem_u32(&empty[s]));
                     }
-                    tc_commit(smem_u32(&empty[s]));
+                    if (ok) tc_commit(smem_u32(&accf[ab]));
                 }
-                if (!ok) {
-                    atomicExch(&fail_s, 1);
-                    break;
-                }
-                tc_commit(smem_u32(&accf[ab]));
+                if (!ok) atomicExch(&fail_s, 1);
             }
             tc_commit(smem_u32(&drained));
             if (!mbar_wait(smem_u32(&drained), 0u)) atomicExch(&fail_s, 1);
         }
+    }
     } else {
-        // ---------------- epilogue (warps 0-3 and 6-9) ----------------
-        // The next tile's view, target rows and row scales are loaded while
-        // the current tile is written back (prep of tile t + 1 before the
-        // wait on tile t's accumulator): the epilogue's per-tile load chains
-        // stay off the path of the reductions.
-        const int ew = warp < 4 ? warp : warp - 2;   // epilogue warp 0..7
+        // ---------------- epilogue (warps 0-7) ----------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TMA_REGS_EPI));
+        // The next segment's row and column scales (and the next tile's
+        // descriptor and target rows) are loaded before the wait on the
+        // current segment's accumulator: their load chains stay off the path
+        // of the reductions.
         const int qw = warp & 3;                       // TMEM lane quarter (rows 32 qw .. 32 qw + 31)
-        const int grp = warp < 4 ? 0 : 1;              // column chunks 32 grp, 32 grp + 64
-        float *E = epi + ew * 32 * 32;
+        const int grp = warp >> 2;                     // column chunks 32 grp, 32 grp + 64
+        float *E = epi + warp * 32 * 32;
         const int myrow = qw * 32 + lane;
-        // two stages: the descriptor of tile t + 2 is loaded while tile t is
-        // written back, and the row targets / scales of tile t + 1 (which need
-        // its descriptor) are requested then too
-        struct EpiTile {
-            TcDesc d;
-            int tr[2];
-            float rs[2], cs[2];
+        struct Scales {
+            float rs[2], cs[2];   // this lane's row of each half; column 32 grp + 64 x + lane
         };
-        auto prep = [&](const TcDesc &d, EpiTile &e) {
-            e.d = d;
-            const bool trsm = (d.flags & 64) != 0;
+        auto scales = [&](const TcDesc &d, int g) {
+            Scales e;
+            e.rs[0] = e.rs[1] = e.cs[0] = e.cs[1] = 1.f;
+            if (F16) {
+                const TcSeg *sg = segs + d.seg0 + g;
+                const int64_t sa = __ldg(&sg->sa) + d.i0, sb = __ldg(&sg->sb) + d.j0;
+                for (int h = 0; h < 2; h++) {
+                    const int r = h * TC_BM + myrow, col = 32 * grp + 64 * h + lane;
+                    e.rs[h] = ((h == 0 || d.pair) && r < d.mrows) ? hscale[sa + r] : 1.f;
+                    e.cs[h] = col < d.ncols ? hscale[sb + col] : 0.f;
+                }
+            }
+            return e;
+        };
+        auto targets = [&](const TcDesc &d, int (&tr)[2]) {
             for (int h = 0; h < 2; h++) {
-                const int row = h * TC_BM + myrow;   // row of the pair, from the first tile's first row
-                const bool ok = (h == 0 || d.pair) && row < d.mrows;
-                e.tr[h] = (ok && !trsm) ? tmap[d.rmap + row] : -1;
-                e.rs[h] = (F16 && ok) ? hscale[d.sa + row] : 1.f;
-                // this warp's two 32-column chunks: column 32 grp + 64 h + lane
-                const int col = 32 * grp + 64 * h + lane;
-                e.cs[h] = (F16 && col < d.ncols) ? hscale[d.sb + col] : 0.f;
+                const int r = h * TC_BM + myrow;
+                tr[h] = ((d.flags & 64) == 0 && (h == 0 || d.pair) && r < d.mrows) ? tmap[d.rmap + r] : -1;
             }
         };
-        EpiTile cur{}, nxt{};
-        TcDesc dn{};
-        if (blockIdx.x < ntiles) prep(tc_desc_load(desc + blockIdx.x), cur);
-        if (blockIdx.x + (int)gridDim.x < ntiles) dn = tc_desc_load(desc + blockIdx.x + gridDim.x);
-        int tl = 0;
-        for (int ti = blockIdx.x; ti < ntiles && !failed(); ti += gridDim.x, tl++) {
-            if (ti + (int)gridDim.x < ntiles) {
-                prep(dn, nxt);
-                if (ti + 2 * (int)gridDim.x < ntiles) dn = tc_desc_load(desc + ti + 2 * gridDim.x);
-            }
-            const TcDesc &v = cur.d;
-            const int ab = tl & 1;
+        TcDesc v{}, vn{};
+        Scales sc{};
+        int trn[2] = {-1, -1};
+        if (blockIdx.x < ntiles) {
+            v = tc_rec_load(desc + blockIdx.x);
+            sc = scales(v, 0);
+            targets(v, trn);
+        }
+        int cnt = 0;
+        bool ok = true;
+        for (int ti = blockIdx.x; ti < ntiles && ok && __all_sync(0xffffffffu, !failed()); ti += gridDim.x) {
+            const bool more = ti + (int)gridDim.x < ntiles;
+            const int trw[2] = {trn[0], trn[1]};   // each lane's row target, shuffled to the writers
+            if (more) vn = tc_rec_load(desc + ti + gridDim.x);
             const bool trsm = (v.flags & 64) != 0;
             const int nh = v.pair ? 2 : 1;
-            if (!mbar_wait(smem_u32(&accf[ab]), (uint32_t)((tl / 2) & 1))) {
-                atomicExch(&fail_s, 1);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int trw[2] = {cur.tr[0], cur.tr[1]};   // each lane's row target, shuffled to the writers
-            const float rs[2] = {cur.rs[0], cur.rs[1]};
-            const float csr[2] = {cur.cs[0], cur.cs[1]};
             float *C = coefL + v.off;
             const int ldf = v.ldo, wf = v.wf;
             const int tcol0 = v.tcol;
             const bool lower_only = (v.flags & 8) != 0;
             const int csh = (v.flags & TC_FLAG_CPLX) ? 1 : 0;
-            // the update subtracts: the sign rides on the row scale
-            const float sgn = trsm ? 1.f : -1.f;
-            for (int h = 0; h < nh; h++)
-            for (int cb = 32 * grp; cb < TC_BN; cb += 64) {
+            // one 32 x 32 chunk (half h, columns cb ..) into the target
+            auto put = [&](int h, int cb, const float (&xx)[32]) {
                 const int mrows = min(TC_BM, v.mrows - h * TC_BM);   // valid rows of this half
-                uint32_t r[32];
-                tc_ld32(tmem + (uint32_t)(ab * 256 + h * 128) + ((uint32_t)(qw * 32) << 16) + (uint32_t)cb, r);
-                __syncwarp();
                 // this lane's row (TMEM lane) as eight 16-byte groups, group g at
                 // slot g ^ (row & 7): conflict-free both for the row-wise stores
                 // here and for the loads along a row / down a column below
-                float x[32];
-                if (F16) {
-                    // column cb + lane's inverse scale (loaded with the tile), broadcast column by column
-                    const float cs = (cb - 32 * grp) ? csr[1] : csr[0], rsh = (h ? rs[1] : rs[0]) * sgn;
-#pragma unroll
-                    for (int q = 0; q < 32; q++) x[q] = __uint_as_float(r[q]) * rsh * __shfl_sync(0xffffffffu, cs, q);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 32; q++) x[q] = __uint_as_float(r[q]) * sgn;
-                }
 #pragma unroll
                 for (int g = 0; g < 8; g++)
                     *reinterpret_cast<float4 *>(E + lane * 32 + ((g ^ (lane & 7)) << 2)) =
-                        make_float4(x[4 * g], x[4 * g + 1], x[4 * g + 2], x[4 * g + 3]);
+                        make_float4(xx[4 * g], xx[4 * g + 1], xx[4 * g + 2], xx[4 * g + 3]);
                 __syncwarp();
                 const int j = cb + lane;
                 if (j < v.ncols && trsm) {
@@ -409,11 +423,89 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
                     }
                 }
                 __syncwarp();
+            };
+            // the update subtracts: the sign rides on the row scale
+            const float sgn = trsm ? 1.f : -1.f;
+            // chunk (h, y) of the accumulator, scaled
+            auto take = [&](int ab, int h, int y, float (&xx)[32], bool more_sums) {
+                uint32_t r[32];
+                tc_ld32(tmem + (uint32_t)(ab * 256 + h * 128) + ((uint32_t)(qw * 32) << 16) +
+                            (uint32_t)(32 * grp + 64 * y), r);
+                const float rsh = (h ? sc.rs[1] : sc.rs[0]) * sgn, csy = y ? sc.cs[1] : sc.cs[0];
+#pragma unroll
+                for (int q = 0; q < 32; q++) {
+                    // column cb + q's inverse scale, broadcast from the lane that holds it
+                    const float p = __uint_as_float(r[q]) * rsh;
+                    const float cs = F16 ? __shfl_sync(0xffffffffu, csy, q) : 1.f;
+                    xx[q] = more_sums ? fmaf(p, cs, xx[q]) : p * cs;
+                }
+            };
+            auto release = [&](int ab) {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&acce[ab]));
+            };
+            auto landed = [&](int n) {
+                if (!mbar_wait_warp(smem_u32(&accf[n & 1]), (uint32_t)((n / 2) & 1))) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                return true;
+            };
+            if (v.nseg == 1) {
+                // a single product: chunk by chunk from the accumulator to the target
+                Scales sn{};
+                if (more) {
+                    sn = scales(vn, 0);
+                    targets(vn, trn);
+                }
+                if (!landed(cnt)) {
+                    atomicExch(&fail_s, 1);
+                    break;
+                }
+                for (int h = 0; h < nh; h++)
+#pragma unroll
+                    for (int y = 0; y < 2; y++) {
+                        const int cb = 32 * grp + 64 * y;
+                        if (cb >= v.ncols) continue;
+                        float xx[32];
+                        take(cnt & 1, h, y, xx, false);
+                        put(h, cb, xx);
+                    }
+                release(cnt & 1);
+                sc = sn;
+                cnt++;
+            } else {
+                float x[2][2][32];   // [half][column chunk][column]
+                for (int g = 0; g < v.nseg; g++, cnt++) {
+                    Scales sn{};
+                    if (g + 1 < v.nseg) {
+                        sn = scales(v, g + 1);
+                    } else if (more) {
+                        sn = scales(vn, 0);
+                        targets(vn, trn);
+                    }
+                    if (!landed(cnt)) {
+                        ok = false;
+                        break;
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+#pragma unroll
+                        for (int y = 0; y < 2; y++)
+                            if (h < nh && 32 * grp + 64 * y < v.ncols) take(cnt & 1, h, y, x[h][y], g > 0);
+                    release(cnt & 1);
+                    sc = sn;
+                }
+                if (!ok) {
+                    atomicExch(&fail_s, 1);
+                    break;
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int y = 0; y < 2; y++)
+                        if (h < nh && 32 * grp + 64 * y < v.ncols) put(h, 32 * grp + 64 * y, x[h][y]);
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&acce[ab]));
-            cur = nxt;
+            v = vn;
         }
     }
     if (tid == 0 && failed()) atomicAdd(&st->timeout, 1);
@@ -578,9 +670,10 @@ __global__ void k_task_rowmap(Meta m, const GemmTask *__restrict__ tasks, const 
 }
 
 // Layout of the FP16 planes: per operand map (mapidx[c] + kind) the first
-// element in the planes (hoff, rows of ld16 halves, a multiple of 8 that holds
-// the row's floats) and the first row in hscale (hsbase).
-__host__ __device__ inline int ld16_of(int nf) { return (nf + 7) & ~7; }
+// element in the planes (hoff, rows of ld16 halves, a multiple of 64 that holds
+// the row's floats, so that no 128-byte box row straddles two lines: 80^3 LU
+// 39.1 -> 38.8 ms) and the first row in hscale (hsbase).
+__host__ __device__ inline int ld16_of(int nf) { return (nf + 63) & ~63; }   // whole 128-byte lines: one per box row
 constexpr int H16_MAXW = 400;   // widest cblk (pastix_gpu_structure)
 
 // The pivots of cblk c (LDL: diagonal of its panel) into shared memory.

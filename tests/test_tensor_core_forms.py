@@ -89,3 +89,40 @@ def test_tensor_core_forms_match_restatement(fact, make, mixed):
     u = 2.0 ** (-24 if mixed else -53)
     assert errs[0] <= 32 * u
     assert errs[0] <= 1.5 * errs[1] + u / 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fact,make", [
+    ("potrf", lambda: M.diffusion_lognormal(40, 37, 39, 1.0, RNG(8))),
+    ("getrf", lambda: M.convdiff_upwind(36, 35, 37, 10.0)),
+    ("hetrf", lambda: M.magnetic_laplacian(33, 34, 32, 0.5, RNG(9))),
+], ids=["potrf", "getrf", "hetrf"])
+def test_fan_in_over_separator_chains(fact, make):
+    """Separators wide enough for chains of several cblks, whose deferred updates are summed before they
+    are scattered: the factor agrees with the FMA tiles', which scatter every source on its own."""
+    from pastix_b200 import autotune as AT
+    from pastix_b200 import gpu as G
+    A = make()
+    st = analysis.analyze(A)
+    s = G.Solver()
+    s.set_iparm(G.IPARM_FACTORIZATION, G.FACT[fact])
+    s.set_iparm(G.IPARM_MIXED, 1)
+    s.set_structure(st)
+    s.set_spm(A)
+    s.numfact(A.values)
+    assert s.stats()["tc_flops"] > 0.8 * s.stats()["gemm_flops"]
+    L, U = s.coeftab()
+    AT.set_knob(s, "mixed_gemm", 0)
+    s.numfact(A.values)
+    L0, U0 = s.coeftab()
+    s.close()
+    lay = NP.Layout(st["cblktab"], st["bloktab"])
+    mask = np.ones(lay.off[-1], bool)
+    if fact != "getrf":
+        for c in range(lay.cblknbr):
+            k = int(lay.width[c])
+            lay.panel(mask, c)[:k, :] &= np.tril(np.ones((k, k), bool))
+    # two single-precision factors of bounded growth, each within a few tens of roundoffs of the exact one
+    for P, Q, m in ((L, L0, mask), (U, U0, None)) if U is not None else ((L, L0, mask),):
+        d, q = (P - Q, Q) if m is None else ((P - Q)[m], Q[m])
+        assert np.linalg.norm(d) <= 64 * 2.0 ** -24 * np.linalg.norm(q)
