@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <queue>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -909,7 +910,8 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     // panels taller than TRSM_GEMM_ROWS: inverse of the diagonal block, then the
     // off-diagonal rows times it as a GEMM (tensor cores in single precision)
     const bool tgemm = !C.record && C.tune[PGPU_TUNE_TRSM_GEMM] != 0;
-    const int key = ((((fmode * 2 + (fp32 ? 1 : 0)) * 2 + (use_tc ? 1 : 0)) * 2 + (zc ? 1 : 0)) * 2 + (tgemm ? 1 : 0));
+    const int key = (((((fmode * 2 + (fp32 ? 1 : 0)) * 2 + (use_tc ? 1 : 0)) * 2 + (zc ? 1 : 0)) * 2 + (tgemm ? 1 : 0)) * 2 +
+                     (C.record ? 1 : 0));
     // (set_tuning invalidates the plan, so the knobs need no place in the key)
     if (C.plan_fact == key) return PASTIX_GPU_SUCCESS;
     invalidate_graph(C);   // the launch lists and workspaces the graph names are rebuilt
@@ -955,7 +957,6 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     std::vector<std::vector<int>> tcl[2];
     for (int k = 0; k < 2; k++) tcl[k].resize(C.nlevels);
     std::vector<std::vector<int>> batches;   // tasks of each batch, the lead first
-    std::vector<int> batch_of;                // lead task -> batch, -1
     // Fan-in (k_gemm_scatter_tc_tma): deferred tasks into the same rows and columns of a cblk, from
     // the successive cblks of a separator chain, are summed in one tile and scattered once, in the
     // level of the last of them.  Keyed by target cblk, columns, panel sides and the rows below.
@@ -1150,8 +1151,6 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             }
         }
     }
-    batch_of.assign(tasks.size(), -1);
-    for (size_t i = 0; i < batches.size(); i++) batch_of[batches[i][0]] = (int)i;
     // their tiles, the deepest sums first (the persistent kernel deals them out in this order)
     for (int l = 0; l < C.nlevels; l++) {
         for (int k = 0; k < 2; k++) {
@@ -1426,9 +1425,15 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
         }
         PGPU_CHECK(C.d_taux.upload(taux, s));
         if (C.tma) {
-            // one segment per task, a batch's contiguous
+            // the segments of a batch's tasks (of a TRSM task), contiguous
             std::vector<TcSeg> segs;
-            std::vector<int> seg0(tasks.size(), -1);
+            std::vector<int> seg0(tasks.size(), -1), nseg(tasks.size(), 0);
+            // k-blocks of a segment (k_gemm_scatter_tc_tma): all of a source in real LL^t and LU, whose sums are as
+            // close as they always were; 64 columns in the LDL and complex forms, whose sums the FMA tiles rounded
+            // to nearest.  Error of the factor, whole depth -> 64 columns (FMA tiles), and of the call's time:
+            // 53x49x61 LDL^t 1.59e-7 -> 1.38e-7 (1.38e-7), 6.36 -> 6.76 ms; complex symmetric 26x27x28 1.27e-7 ->
+            // 1.23e-7 (1.21e-7), 60^3 complex LDL^h 21.8 -> 23.0 ms
+            const int seg_nk = C.h16 && (zc || ldl) ? cs : INT_MAX;
             auto add_seg = [&](int id) {
                 const GemmTask &g = tasks[id];
                 const bool trsm = (g.flags & 64) != 0;
@@ -1442,22 +1447,25 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 e.mapb = mb + kb;
                 e.rowa = g.arow0;
                 e.rowb = cs * (trsm ? 0 : C.browoff[g.b]);
-                e.nk = cdiv(cs * C.width[g.c], C.h16 ? 64 : TC_BK);
                 if (C.h16) {
                     e.sa = hsbase_h[mb + ka] + e.rowa;
                     e.sb = hsbase_h[mb + kb] + e.rowb;
                 }
-                segs.push_back(e);
-            };
-            for (const auto &bt : batches) {
-                seg0[bt[0]] = (int)segs.size();
-                for (int id : bt) add_seg(id);
-            }
-            for (const int4 &t : tttiles)
-                if (seg0[t.x] < 0) {
-                    seg0[t.x] = (int)segs.size();
-                    add_seg(t.x);
+                const int nk = cdiv(cs * C.width[g.c], C.h16 ? 64 : TC_BK), parts = cdiv(nk, seg_nk);
+                for (int q = 0; q < parts; q++) {
+                    e.kb0 = (int)((int64_t)nk * q / parts);
+                    e.nk = (int)((int64_t)nk * (q + 1) / parts) - e.kb0;
+                    segs.push_back(e);
                 }
+            };
+            auto add_tile = [&](int lead, const std::vector<int> &ids) {
+                seg0[lead] = (int)segs.size();
+                for (int id : ids) add_seg(id);
+                nseg[lead] = (int)segs.size() - seg0[lead];
+            };
+            for (const auto &bt : batches) add_tile(bt[0], bt);
+            for (const int4 &t : tttiles)
+                if (seg0[t.x] < 0) add_tile(t.x, {t.x});
             PGPU_CHECK(C.d_tcseg.upload(segs, s));
             // one descriptor per tensor-core tile (k_gemm_scatter_tc_tma reads no task tables)
             auto make_desc = [&](const int4 &t) {
@@ -1469,7 +1477,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                 TcDesc d;
                 std::memset(&d, 0, sizeof(d));
                 d.seg0 = seg0[t.x];
-                d.nseg = trsm ? 1 : (int)batches[batch_of[t.x]].size();
+                d.nseg = nseg[t.x];
                 d.ncols = std::min(TC_BN, N - j0);
                 d.pair = t.w & 1;
                 d.flags = g.flags | (zc ? TC_FLAG_CPLX : 0);
@@ -1651,6 +1659,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
     // split products (3xTF32; the 3xFP16 mode without TMA operands falls back to it)
     const bool split = (mixed_gemm_mode(C) == MG_3XTF32 || mixed_gemm_mode(C) == MG_3XF16);
     const bool persist = C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record;   // task timings need one tile per CTA
+    if (C.tma && !persist) return PASTIX_GPU_ERR_INTERNAL;   // (its tile lists are leads of batches, and pairs)
     int nsm = 148;
     if constexpr (F32) {
         PGPU_CHECK(cudaFuncSetAttribute(k_gemm_scatter_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -87,12 +87,16 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
 // reductions into the target panel, which bound the kernel when every source
 // writes its own (100^3: 41 GB of them), shrink by the number of segments.  A
 // tile of one segment goes chunk by chunk from the accumulator to the target
-// (through the registers of a whole tile it took a third longer).  With the
+// (through the registers of a whole tile it took a third longer).
+// A segment may also be a part of its source's columns: the tensor core's
+// additions cut off what lies below the accumulator's last bits, always
+// towards zero, so that the error of a sum grows with its length faster than
+// that of an FMA chain; the additions in the epilogue round to nearest.  With the
 // fan-in what bounds the kernel is the latency of its loads: on 72^3, tensor
 // pipe 43 % of active cycles, L2 23 %, DRAM below 15 %.
 struct __align__(16) TcSeg {
     int mapa, mapb, rowa, rowb;   // tensor maps (indices into maps), first row of the task in A and in B
-    int nk, pad[3];               // k-blocks
+    int nk, kb0, pad[2];          // k-blocks, the first of them
     int64_t sa, sb;               // 3xFP16: scale index of those rows
 };
 struct __align__(16) TcDesc {
@@ -211,9 +215,9 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
                             break;
                         }
                         mbar_arrive_expect_tx(smem_u32(&full[s]), bytes);
-                        tma_load_3d(tile_addr(s, 0), ma, kb * BK, rowa, 0, smem_u32(&full[s]));
-                        if (o.pair) tma_load_3d(tile_addr(s, QA1), ma, kb * BK, rowa + TC_BM, 0, smem_u32(&full[s]));
-                        tma_load_3d(tile_addr(s, QB), mbm, kb * BK, rowb, 0, smem_u32(&full[s]));
+                        tma_load_3d(tile_addr(s, 0), ma, (sg.kb0 + kb) * BK, rowa, 0, smem_u32(&full[s]));
+                        if (o.pair) tma_load_3d(tile_addr(s, QA1), ma, (sg.kb0 + kb) * BK, rowa + TC_BM, 0, smem_u32(&full[s]));
+                        tma_load_3d(tile_addr(s, QB), mbm, (sg.kb0 + kb) * BK, rowb, 0, smem_u32(&full[s]));
                     }
                 }
                 if (!ok) atomicExch(&fail_s, 1);
@@ -426,19 +430,27 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
             };
             // the update subtracts: the sign rides on the row scale
             const float sgn = trsm ? 1.f : -1.f;
-            // chunk (h, y) of the accumulator, scaled
+            // chunk (h, y) of the accumulator, scaled.  Every lane needs every column's scale: they go through
+            // the warp's buffer, read back as 16-byte broadcasts
             auto take = [&](int ab, int h, int y, float (&xx)[32], bool more_sums) {
+                if (F16) E[lane] = y ? sc.cs[1] : sc.cs[0];
                 uint32_t r[32];
                 tc_ld32(tmem + (uint32_t)(ab * 256 + h * 128) + ((uint32_t)(qw * 32) << 16) +
                             (uint32_t)(32 * grp + 64 * y), r);
-                const float rsh = (h ? sc.rs[1] : sc.rs[0]) * sgn, csy = y ? sc.cs[1] : sc.cs[0];
+                __syncwarp();
+                const float rsh = (h ? sc.rs[1] : sc.rs[0]) * sgn;
 #pragma unroll
-                for (int q = 0; q < 32; q++) {
-                    // column cb + q's inverse scale, broadcast from the lane that holds it
-                    const float p = __uint_as_float(r[q]) * rsh;
-                    const float cs = F16 ? __shfl_sync(0xffffffffu, csy, q) : 1.f;
-                    xx[q] = more_sums ? fmaf(p, cs, xx[q]) : p * cs;
+                for (int q = 0; q < 32; q += 4) {
+                    float4 c = make_float4(1.f, 1.f, 1.f, 1.f);
+                    if (F16) c = *reinterpret_cast<const float4 *>(E + q);
+                    const float cs[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const float p = __uint_as_float(r[q + u]) * rsh;
+                        xx[q + u] = more_sums ? fmaf(p, cs[u], xx[q + u]) : p * cs[u];
+                    }
                 }
+                __syncwarp();
             };
             auto release = [&](int ab) {
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

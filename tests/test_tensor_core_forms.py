@@ -126,3 +126,58 @@ def test_fan_in_over_separator_chains(fact, make):
     for P, Q, m in ((L, L0, mask), (U, U0, None)) if U is not None else ((L, L0, mask),):
         d, q = (P - Q, Q) if m is None else ((P - Q)[m], Q[m])
         assert np.linalg.norm(d) <= 64 * 2.0 ** -24 * np.linalg.norm(q)
+
+
+# --- sums of the LDL and complex forms -----------------------------------------
+def _lower(st):
+    lay = NP.Layout(st["cblktab"], st["bloktab"])
+    mask = np.ones(lay.off[-1], bool)
+    for c in range(lay.cblknbr):
+        k = int(lay.width[c])
+        lay.panel(mask, c)[:k, :] &= np.tril(np.ones((k, k), bool))
+    return mask
+
+
+def _mixed_factors(A, st, fact):
+    """Single-precision factor on the tensor cores and on the FMA tiles."""
+    from pastix_b200 import autotune as AT
+    from pastix_b200 import gpu as G
+    s = G.Solver()
+    s.set_iparm(G.IPARM_FACTORIZATION, G.FACT[fact])
+    s.set_iparm(G.IPARM_MIXED, 1)
+    s.set_structure(st)
+    s.set_spm(A)
+    s.numfact(A.values)
+    stats = s.stats()
+    assert stats["tc_flops"] > 0.7 * stats["gemm_flops"]
+    out = [s.coeftab()]
+    AT.set_knob(s, "mixed_gemm", 0)
+    s.numfact(A.values)
+    out.append(s.coeftab())
+    s.close()
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fact,make,spread", [
+    ("sytrf", lambda: M.diffusion_lognormal(44, 43, 45, 1.0, RNG(8)), 1.08),
+    ("sytrf", lambda: _csym(M.diffusion_lognormal(30, 29, 31, 1.0, RNG(4)), 5), 1.04),
+], ids=["sytrf", "sytrf_z"])
+def test_ldl_sums_are_as_close_as_the_fma_tiles(fact, make, spread):
+    """Terms of one sign, over sources of up to some 200 columns: the tensor core's additions cut off, the FMA
+    tiles' round to nearest, everything else is the same.  Errors against the 64-bit factor.  `spread`: the real
+    form keeps its operands' 22 bits and the twelve cut-off additions of 64 columns, of 6 units 2^-25 of a sum
+    beside the FMA chain's 4 to 5 (sums cut off over the whole depth: 1.18 of the FMA tiles' error, complex 1.06)."""
+    from pastix_b200 import gpu as G
+    A = make()
+    st = analysis.analyze(A)
+    s = G.Solver()
+    s.set_iparm(G.IPARM_FACTORIZATION, G.FACT[fact])
+    s.set_structure(st)
+    s.set_spm(A)
+    s.numfact(A.values)
+    L0, _ = s.coeftab()
+    s.close()
+    m = _lower(st)
+    e_tc, e_fma = (np.linalg.norm((L - L0)[m]) for L, _ in _mixed_factors(A, st, fact))
+    assert e_tc <= spread * e_fma
