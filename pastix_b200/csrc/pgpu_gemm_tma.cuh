@@ -109,6 +109,10 @@ struct __align__(16) TcDesc {
 };
 static_assert(sizeof(TcSeg) == 48 && sizeof(TcDesc) == 64, "whole 16-byte vectors");
 
+// 2^e, and e of 2^e, for normal floats.
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
+__device__ __forceinline__ int pow2_exp(float x) { return (__float_as_int(x) >> 23) - 127; }
+
 template <typename R>
 __device__ __forceinline__ R tc_rec_load(const R *p) {
     R d;
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
                 for (int h = 0; h < 2; h++) {
                     const int r = h * TC_BM + myrow, col = 32 * grp + 64 * h + lane;
                     e.rs[h] = ((h == 0 || d.pair) && r < d.mrows) ? hscale[sa + r] : 1.f;
-                    e.cs[h] = col < d.ncols ? hscale[sb + col] : 0.f;
+                    e.cs[h] = col < d.ncols ? hscale[sb + col] : 1.f;
                 }
             }
             return e;
@@ -452,6 +456,19 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
                 }
                 __syncwarp();
             };
+            // An accumulator reaches 2^40: a row scale above 2^60 hands what it has beyond to the columns', so that
+            // the product with the row scale stays in range where the product with both does (powers of two:
+            // exact but for rows 2^130 below others of their 32)
+            auto balance = [&]() {
+                if (!F16 || !__any_sync(0xffffffffu, fmaxf(sc.rs[0], sc.rs[1]) > 0x1p60f)) return;
+                const int re = __reduce_max_sync(0xffffffffu, pow2_exp(fmaxf(sc.rs[0], sc.rs[1])));
+                const int ce = __reduce_max_sync(0xffffffffu, pow2_exp(fmaxf(sc.cs[0], sc.cs[1])));
+                const int t = max(0, min(re - 60, 120 - ce));
+                for (int h = 0; h < 2; h++) {
+                    sc.rs[h] *= pow2f(-t);
+                    sc.cs[h] *= pow2f(t);
+                }
+            };
             auto release = [&](int ab) {
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -473,6 +490,7 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
                     atomicExch(&fail_s, 1);
                     break;
                 }
+                balance();
                 for (int h = 0; h < nh; h++)
 #pragma unroll
                     for (int y = 0; y < 2; y++) {
@@ -499,6 +517,7 @@ __global__ void __launch_bounds__(TMA_THREADS, 1)
                         ok = false;
                         break;
                     }
+                    balance();
 #pragma unroll
                     for (int h = 0; h < 2; h++)
 #pragma unroll
@@ -564,7 +583,6 @@ __global__ void k_split_rows(Meta m, const int4 *__restrict__ jobs, const float 
 // maximum 65504 and far above its normal minimum 2^-14.  e is clamped to
 // [-126, 126] so that 2^e and 2^-e are normal floats (an all-zero row keeps
 // e = 0).  The row's stored scale is 2^-e, which the GEMM epilogue applies.
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
 
 // One warp splits one row of nf floats (complex: interleaved parts; src 16-byte
 // aligned, padded to a multiple of 4): optionally times dsc (one factor per

@@ -181,3 +181,30 @@ def test_ldl_sums_are_as_close_as_the_fma_tiles(fact, make, spread):
     m = _lower(st)
     e_tc, e_fma = (np.linalg.norm((L - L0)[m]) for L, _ in _mixed_factors(A, st, fact))
     assert e_tc <= spread * e_fma
+
+
+def _times(A, f):
+    A.values = A.values * f
+    return A
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fact,make", [
+    ("sytrf", lambda: _times(M.diffusion_lognormal(20, 17, 19, 0.3, RNG(2)), 1e36)),
+    ("hetrf", lambda: _times(M.magnetic_laplacian(20, 19, 18, -0.5, RNG(3)), 1e35)),
+    ("getrf", lambda: _times(_phased(M.convdiff_upwind(15, 14, 16, 10.0), 6), 1e35)),
+    ("sytrf", lambda: _times(M.diffusion_lognormal(20, 17, 19, 0.3, RNG(2)), 1e-30)),
+], ids=["sytrf_1e36", "hetrf_1e35", "getrf_z_1e35", "sytrf_1e-30"])
+def test_matrices_of_extreme_scale(fact, make):
+    """Rows near the largest float: an accumulator times one of its two scales leaves the range, the result
+    does not.  The FMA tiles take these matrices, so the tensor cores have to."""
+    A = make()
+    st = analysis.analyze(A)
+    (L, U), (L0, U0) = _mixed_factors(A, st, fact)
+    m = _lower(st) if fact != "getrf" else np.ones(L.size, bool)
+    for P, Q, k in ((L, L0, m),) + (((U, U0, m),) if U is not None else ()):
+        q = Q[k].astype(np.complex128)
+        d = P[k].astype(np.complex128) - q
+        t = np.abs(q).max()
+        # (as between the two in test_fan_in_over_separator_chains)
+        assert np.linalg.norm(d / t) <= 64 * 2.0 ** -24 * np.linalg.norm(q / t)
