@@ -2171,11 +2171,9 @@ extern "C" int pastix_gpu_numfact(pastix_gpu_t *ctx, const void *values) {
     C.stats[12] = C.tc_flops;   // tensor-core (tcgen05, or FP64 DMMA) task flops
     C.stats[13] = st.timeout;
     C.stats[14] = replayed ? 1.0 : 0.0;
-    if (st.timeout || st.drain_timeout) {
-        fprintf(stderr, "pastix_gpu: %d tensor-core GEMM tiles timed out waiting for their MMAs\n", st.timeout);
-        if (st.drain_timeout)
-            fprintf(stderr, "pastix_gpu: %d CTAs gave up waiting for their own TMA loads after a time-out: the "
-                            "factorization's results are undefined\n", st.drain_timeout);
+    const std::string timeouts = status_timeouts(st);
+    if (!timeouts.empty()) {
+        fputs(timeouts.c_str(), stderr);
         C.fact_done = -1;
         return PASTIX_GPU_ERR_INTERNAL;
     }

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <string>
 #include <type_traits>
 
 namespace pgpu {
@@ -54,10 +55,26 @@ struct Status {
     int negpivots;     // negative/zero diagonal met in a Cholesky pivot
     int nonfinite;     // NaN/Inf met on a diagonal
     int overflow;      // FP32 down-cast overflow in the mixed fill-in
-    int timeout;       // a bounded wait inside a kernel gave up (tile skipped)
+    int timeout;       // a bounded wait of a tensor-core GEMM kernel gave up (tile skipped)
+    int panel_timeout; // one of the diagonal blocks' kernels gave up (k_panel_rows, k_tri_inverse)
     int drain_timeout; // after a time-out, waiting for a CTA's own TMA loads in flight gave up too: the
                        // launch's results are undefined (its shared memory may still receive those bytes)
 };
+
+// The time-outs of a status, in words, one line each; empty: none.
+inline std::string status_timeouts(const Status &st) {
+    std::string s;
+    if (st.timeout)
+        s += "pastix_gpu: " + std::to_string(st.timeout) + " CTAs' tensor-core GEMM tiles timed out waiting for their "
+             "loads or MMAs\n";
+    if (st.panel_timeout)
+        s += "pastix_gpu: " + std::to_string(st.panel_timeout) + " CTAs timed out in the diagonal blocks, waiting for "
+             "an earlier block row or for their loads (a block row that gives up takes those behind it along)\n";
+    if (st.drain_timeout)
+        s += "pastix_gpu: " + std::to_string(st.drain_timeout) + " CTAs gave up waiting for their own loads in flight "
+             "after a time-out: the factorization's results are undefined\n";
+    return s;
+}
 
 // Complex scalar (interleaved re, im: the layout of pastix_complex64_t /
 // pastix_complex32_t and of C99 double/float _Complex).

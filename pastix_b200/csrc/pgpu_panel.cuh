@@ -481,7 +481,7 @@ __host__ __device__ inline size_t tri_inverse_lb_offset(int nrow, size_t esz) {
 // PB rows x bulk_lb (strip) and PB rows x (PB + VK) (tile): the copies of
 // the next tile row are in flight while the current one is computed.  A
 // copy that does not land within the bounded wait is counted in
-// Status::timeout and the factorization reported failed.
+// Status::panel_timeout and the factorization reported failed.
 template <typename T>
 __global__ void __launch_bounds__(256) k_tri_inverse(Meta m, const int2 *__restrict__ jobs,
                                                      const T *__restrict__ coefL, T *__restrict__ inv,
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(256) k_tri_inverse(Meta m, const int2 *__restr
             if (tfail) {
                 if (tid == 0) {
                     // this step's copies and, when issued, the next step's land before the CTA leaves
-                    atomicAdd(&st->timeout, 1);
+                    atomicAdd(&st->panel_timeout, 1);
                     if (!mbar_wait(smem_u32(&tmb[b]), (uint32_t)((stp >> 1) & 1))) atomicAdd(&st->drain_timeout, 1);
                     if (ib + PB < w && !mbar_wait(smem_u32(&tmb[b ^ 1]), (uint32_t)(((stp + 1) >> 1) & 1)))
                         atomicAdd(&st->drain_timeout, 1);

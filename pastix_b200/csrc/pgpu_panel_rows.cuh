@@ -19,7 +19,7 @@
 // inverse CTA (column block j) waits row by row: Inv_ij = -T_i sum_m L_im
 // Inv_mj with T_i the tile's inverse.  CTAs take their jobs from a ticket in an
 // order where a job waits only for earlier ones, so whatever part of the
-// launch is resident makes progress.  All waits are bounded (Status::timeout).
+// launch is resident makes progress.  All waits are bounded (Status::panel_timeout).
 //
 // What bounds it: the chain of w / 32 steps, each one L2 round trip (poll and
 // tile), two 32^3 products, and the 32-column elimination of the tile on one
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
             }
         }
     }
-    if (tid == 0 && failed()) atomicAdd(&st->timeout, 1);
+    if (tid == 0 && failed()) atomicAdd(&st->panel_timeout, 1);
 }
 
 }  // namespace pgpu
