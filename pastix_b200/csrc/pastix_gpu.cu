@@ -135,6 +135,7 @@ struct pastix_gpu_s {
     // lvl_cblks} (the position indexes the task records)
     std::vector<int> pn_ptr, lvl_pmaxw;
     DArr<int2> d_pjobs;
+    DArr<int> d_cblkpos;   // while recording: each cblk's position in lvl_cblks
     // diagonal blocks taken one CTA per block row (k_panel_rows): jobs, and per
     // level the staging slots and shared memory of its widest block; counters
     // (one per block row of the plan, then one ticket per level), published tiles
@@ -694,7 +695,7 @@ static int fact_mode_of(int fact, bool zc) {
 const int PR_FEW = 592;
 static bool rows_panel(const pastix_gpu_t &C, int w, size_t esz, bool lu, int nlvl) {
     const int64_t wmin = C.tune[PGPU_TUNE_WIDE_PANEL];
-    return wmin > 0 && !C.record && w > PB && (w >= wmin || nlvl <= PR_FEW) && pr_slots(w, esz, lu, WP_SMEM_LIMIT) > 0;
+    return wmin > 0 && w > PB && (w >= wmin || nlvl <= PR_FEW) && pr_slots(w, esz, lu, WP_SMEM_LIMIT) > 0;
 }
 
 // Forget the captured factorization graph (its nodes name the plan's and the
@@ -1581,7 +1582,8 @@ enum { PH_DIAG = 0, PH_TRSM = 1, PH_GEMM = 2, PH_TC = 3, PH_END = 4 };
 template <typename T>
 using PanelKernel = void (*)(Meta, const int2 *, T *, T *, const double *, int, int, int, Status *, int64_t *);
 template <typename T>
-using RowsKernel = void (*)(Meta, const int4 *, int *, int *, T *, T *, T *, T *, const double *, int, int, Status *);
+using RowsKernel = void (*)(Meta, const int4 *, int *, int *, T *, T *, T *, T *, const double *, int, int, Status *,
+                            const int *, int64_t *);
 
 template <typename T>
 using SmallPanelKernel = void (*)(Meta, const int2 *, int, T *, T *, const double *, int, Status *);
@@ -1687,6 +1689,12 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
             if (C.d_prof[k].n < 2 * cnt[k]) PGPU_CHECK(C.d_prof[k].alloc(2 * cnt[k]));
             prof[k] = cnt[k] ? C.d_prof[k].p : nullptr;
         }
+        // (a panel's block rows each raise its end)
+        PGPU_CHECK(cudaMemsetAsync(C.d_prof[0].p, 0, 2 * cnt[0] * sizeof(int64_t), s));
+        std::vector<int> pos(C.cblknbr);
+        for (int q = 0; q < C.cblknbr; q++) pos[C.lvl_cblks[q]] = q;
+        PGPU_CHECK(C.d_cblkpos.upload(pos, s));
+        PGPU_CHECK(cudaStreamSynchronize(s));   // (pos leaves scope)
     }
     auto at = [](int64_t *p, int off) { return p ? p + 2 * (int64_t)off : nullptr; };
     const double *critp = C.d_fact_scal.p + 1;
@@ -1820,7 +1828,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
             krows<<<npr, PR_THREADS, C.pr_lsmem[l], s>>>(
                 C.meta, C.d_prjobs.p + C.pr_ptr[l], C.d_prog.p + C.pr_counters + l, C.d_prog.p,
                 reinterpret_cast<T *>(C.d_prscr.p), coefL, coefU, reinterpret_cast<T *>(C.d_inv.p), critp, fuse,
-                C.pr_lslots[l], C.d_status.p);
+                C.pr_lslots[l], C.d_status.p, C.d_cblkpos.p, prof[0]);
             nl++;
         }
         if constexpr (sizeof(T) <= 8) {

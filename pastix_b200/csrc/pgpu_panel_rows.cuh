@@ -258,7 +258,7 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_rows(Meta m, const int4 *__restrict__ jobs, int *ticket,
                                                            int *prog, T *scr, T *coefL, T *coefU, T *inv,
                                                            const double *critp, int fuse_rows, int slots,
-                                                           Status *st) {
+                                                           Status *st, const int *pos, int64_t *prof) {
     typedef typename real_of<T>::type R;
     constexpr bool LU = (MODE == FM_GETRF), LDL = fm_ldl(MODE), CJ = fm_conj(MODE);
     constexpr int VK = pr_vk<T>(), P = pr_pitch<T>(), TILE = pr_tile<T>(), NV = PB / VK;
@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
     __syncthreads();
     const int4 jb = jobs[job_s];
     const int c = jb.x, kind = jb.y >> 16, i = jb.y & 0xffff;
+    const uint64_t t_start = prof ? global_ns() : 0;
     const int w = m.width[c], h = m.height[c], ld = m.ld[c];
     const int nt = (w + PB - 1) / PB;
     T *A = coefL + m.coefoff[c], *AU = coefU + m.coefoff[c];
@@ -536,6 +537,15 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
         }
     }
     if (tid == 0 && failed()) atomicAdd(&st->panel_timeout, 1);
+    if (prof && kind == PR_ROW) {
+        // the panel's task record: from the start of its first block row to the end of its last
+        __syncthreads();
+        if (tid == 0) {
+            int64_t *t = prof + 2 * (int64_t)pos[c];
+            if (i == 0) t[0] = (int64_t)t_start;
+            atomicMax(reinterpret_cast<unsigned long long *>(t + 1), (unsigned long long)global_ns());
+        }
+    }
 }
 
 }  // namespace pgpu
