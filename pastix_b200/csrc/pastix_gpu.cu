@@ -38,6 +38,7 @@ using namespace pgpu;
         if (e_ != cudaSuccess) {                                                       \
             fprintf(stderr, "pastix_gpu: %s failed: %s (%s:%d)\n", #x,                 \
                     cudaGetErrorString(e_), __FILE__, __LINE__);                       \
+            (void)cudaGetLastError(); /* (reported: not the next call's error) */      \
             return e_ == cudaErrorMemoryAllocation ? PASTIX_GPU_ERR_OUTOFMEMORY        \
                                                    : PASTIX_GPU_ERR_INTERNAL;          \
         }                                                                              \
@@ -2143,6 +2144,9 @@ extern "C" int pastix_gpu_numfact(pastix_gpu_t *ctx, const void *values) {
             cudaGraph_t g = nullptr;
             const cudaError_t ec = cudaStreamEndCapture(s, &g);
             if (rc) {
+                // (a call refused half-way leaves the second stream unjoined: the capture ends with that error,
+                // which the next call of any kind must not find)
+                (void)cudaGetLastError();
                 if (g) cudaGraphDestroy(g);
                 return rc;
             }
