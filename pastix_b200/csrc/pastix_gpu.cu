@@ -52,9 +52,11 @@ struct DArr {
     size_t n = 0;
     cudaError_t alloc(size_t cnt) {
         release();
-        n = cnt;
         if (!cnt) return cudaSuccess;
-        return cudaMalloc(&p, cnt * sizeof(T));
+        const cudaError_t e = cudaMalloc(&p, cnt * sizeof(T));
+        if (e == cudaSuccess) n = cnt;   // (a failed one must not look large enough to the next call)
+        else p = nullptr;
+        return e;
     }
     cudaError_t upload(const std::vector<T> &v, cudaStream_t s) {
         cudaError_t e = alloc(v.size());

@@ -1,0 +1,76 @@
+"""Plans when device memory is short."""
+import contextlib
+
+import numpy as np
+import pytest
+
+from pastix_b200 import analysis
+from pastix_b200 import matrices as M
+
+RNG = np.random.default_rng
+
+
+def _solver(A, st, fact, mixed=1, **knobs):
+    from pastix_b200 import autotune as AT
+    from pastix_b200 import gpu as G
+    s = G.Solver()
+    s.set_iparm(G.IPARM_FACTORIZATION, G.FACT[fact])
+    s.set_iparm(G.IPARM_MIXED, mixed)
+    s.set_structure(st)
+    s.set_spm(A)
+    for k, v in knobs.items():
+        AT.set_knob(s, k, v)
+    return s
+
+
+def _free():
+    import torch
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _takes(A, st, fact, **knobs):
+    """Device memory a first factorization and solve take (the second of two handles: kernels are loaded)."""
+    x, b = M.rhs_from_xtrue(A, 1, RNG(1))
+    for _ in range(2):
+        s = _solver(A, st, fact, **knobs)
+        f0 = _free()
+        s.numfact(A.values)
+        s.solve(b)
+        used = f0 - _free()
+        s.close()
+    return used
+
+
+@contextlib.contextmanager
+def _only(room):
+    """All of the device's memory but `room` bytes taken."""
+    import torch
+    hog = torch.empty(_free() - room, dtype=torch.uint8, device="cuda")
+    yield
+    del hog
+    _free()
+
+
+def _check(s, A):
+    x, b = M.rhs_from_xtrue(A, 1, RNG(1))
+    assert np.linalg.norm(s.solve(b) - x) <= 1e-4 * np.linalg.norm(x)
+    return s.stats()["tc_flops"]
+
+
+@pytest.mark.gpu
+def test_a_failed_allocation_is_made_good():
+    """A factorization without room is refused, and the next one, with room, allocates what it lacks."""
+    from pastix_b200 import gpu as G
+    A = M.diffusion_lognormal(30, 29, 31, 1.0, RNG(2))
+    st = analysis.analyze(A)
+    _takes(A, st, "potrf")                                   # (kernels loaded)
+    s = _solver(A, st, "potrf", mixed=0)
+    with _only(16 * 2 ** 20):
+        with pytest.raises(G.PastixGpuError) as e:
+            s.numfact(A.values)
+        assert e.value.code == 4
+    s.numfact(A.values)
+    _check(s, A)
+    s.close()
