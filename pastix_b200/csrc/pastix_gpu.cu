@@ -918,6 +918,8 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
                      (C.record ? 1 : 0));
     // (set_tuning invalidates the plan, so the knobs need no place in the key)
     if (C.plan_fact == key) return PASTIX_GPU_SUCCESS;
+    C.plan_fact = -1;      // (a plan that fails half-way is nobody's,
+    C.fact_done = -1;      // and the factor at hand loses its inverses and solve lists to the new one)
     invalidate_graph(C);   // the launch lists and workspaces the graph names are rebuilt
     const size_t esz = (fp32 ? 4 : 8) * (zc ? 2 : 1);
     const int fuse = tgemm ? std::min((int)C.tune[PGPU_TUNE_TRSM_GEMM_ROWS], fuse_rows_for(lu, esz))

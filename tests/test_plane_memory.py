@@ -74,3 +74,24 @@ def test_a_failed_allocation_is_made_good():
     s.numfact(A.values)
     _check(s, A)
     s.close()
+
+
+@pytest.mark.gpu
+def test_a_plan_that_fails_leaves_no_factor():
+    """Its solve lists and inverses belong half to the plan that was not finished."""
+    from pastix_b200 import gpu as G
+    A = M.diffusion_lognormal(30, 29, 31, 1.0, RNG(2))
+    st = analysis.analyze(A)
+    room = _takes(A, st, "potrf") // 4
+    s = _solver(A, st, "potrf")
+    s.numfact(A.values)
+    s.set_iparm(G.IPARM_MIXED, 0)
+    with _only(room):
+        with pytest.raises(G.PastixGpuError):
+            s.numfact(A.values)
+        with pytest.raises(G.PastixGpuError):
+            s.solve(np.ones(A.n))
+    s.set_iparm(G.IPARM_MIXED, 1)
+    s.numfact(A.values)
+    assert _check(s, A) > 0
+    s.close()
