@@ -208,7 +208,6 @@ struct pastix_gpu_s {
     // coeftab and of the inverses (3xTF32), one tensor map per (source cblk,
     // operand kind), split jobs {cblk, row, panel, -} per level
     bool tma = false;
-    bool tma_failed = false, forms_off = false;   // no tensor maps; no room for the LDL / complex planes
     DArr<float> d_hilo, d_ihilo;
     // 3xFP16 operands (mixed GEMM mode 3): FP16 hi / lo planes [2][h16_plane]
     // of the source matrices, per-row inverse scales, and per operand map its
@@ -465,7 +464,6 @@ extern "C" int pastix_gpu_structure(pastix_gpu_t *ctx, int64_t n, int64_t cblknb
     }
     PGPU_CHECK(C.d_solve_chunks.upload(sch, s));
     C.plan_fact = -1;
-    C.tma_failed = C.forms_off = false;
     C.fact_done = -1;
     C.d_coef.release();
     PGPU_CHECK(cudaStreamSynchronize(s));
@@ -896,11 +894,18 @@ static int build_flow_plan(pastix_gpu_t &C, size_t esz, bool lu) {
     return flow_reset(C);
 }
 
-static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
+// What a plan may use: no tensor maps (the encoder refused one), no room for the LDL / complex planes.
+// Found while the plan is made, which starts again without it; the next plan tries everything anew.
+struct PlanRoute {
+    bool tma = true, forms = true;
+};
+
+// (*again: `route` has been narrowed, make the plan again)
+static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRoute &route, bool *again) {
     // single precision: the large update and TRSM GEMMs on the tcgen05 tensor cores; the LDL and the
     // complex forms only as 3xFP16 with pre-split operands (D and the complex product live in the planes)
     const bool h16_forms = fp32 && mixed_gemm_mode(C) == MG_3XF16 && C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record &&
-                           C.tune[PGPU_TUNE_TC_TMA] != 0 && tensor_map_encoder() != nullptr && !C.tma_failed && !C.forms_off;
+                           C.tune[PGPU_TUNE_TC_TMA] != 0 && tensor_map_encoder() != nullptr && route.tma && route.forms;
     const bool use_tc = fp32 && tc_enabled(C) && ((!zc && (fmode == FM_POTRF || fmode == FM_GETRF)) || h16_forms);
     const int cs = zc ? 2 : 1;   // floats per element: the tensor-core tiles of complex tasks are real ones
     // FP64: the large update and TRSM GEMMs on the FP64 tensor cores (DMMA),
@@ -914,13 +919,6 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     // panels taller than TRSM_GEMM_ROWS: inverse of the diagonal block, then the
     // off-diagonal rows times it as a GEMM (tensor cores in single precision)
     const bool tgemm = !C.record && C.tune[PGPU_TUNE_TRSM_GEMM] != 0;
-    const int key = (((((fmode * 2 + (fp32 ? 1 : 0)) * 2 + (use_tc ? 1 : 0)) * 2 + (zc ? 1 : 0)) * 2 + (tgemm ? 1 : 0)) * 2 +
-                     (C.record ? 1 : 0));
-    // (set_tuning invalidates the plan, so the knobs need no place in the key)
-    if (C.plan_fact == key) return PASTIX_GPU_SUCCESS;
-    C.plan_fact = -1;      // (a plan that fails half-way is nobody's,
-    C.fact_done = -1;      // and the factor at hand loses its inverses and solve lists to the new one)
-    invalidate_graph(C);   // the launch lists and workspaces the graph names are rebuilt
     const size_t esz = (fp32 ? 4 : 8) * (zc ? 2 : 1);
     const int fuse = tgemm ? std::min((int)C.tune[PGPU_TUNE_TRSM_GEMM_ROWS], fuse_rows_for(lu, esz))
                            : fuse_rows_for(lu, esz);
@@ -968,7 +966,7 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     // level of the last of them.  Keyed by target cblk, columns, panel sides and the rows below.
     const bool tma_mode = use_tc && (mixed_gemm_mode(C) == MG_3XTF32 || mixed_gemm_mode(C) == MG_3XF16) &&
                           C.tune[PGPU_TUNE_TC_KERNEL] != 0 && !C.record && C.tune[PGPU_TUNE_TC_TMA] != 0 &&
-                          tensor_map_encoder() != nullptr && !C.tma_failed;
+                          tensor_map_encoder() != nullptr && route.tma;
     struct FanKey {
         int f, r0, r1, flags, M;
         uint64_t tail;
@@ -1231,13 +1229,16 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             // (complex planes are three times the factor: where they do not fit beside it, FMA tiles)
             size_t mfree = 0, mtotal = 0;
             PGPU_CHECK(cudaMemGetInfo(&mfree, &mtotal));
-            auto more = [](size_t want, size_t have) { return want > have ? want : 0; };
+            auto more = [](size_t want, size_t have) { return want > have ? want - have : 0; };
+            const size_t vec = (size_t)C.n * flow_maxrhs(esz) * esz;   // the dataflow solve's Y, Z
             const size_t need = more(4 * (size_t)C.h16_plane, C.d_h16.n * 2) +
                                 more((size_t)C.coefnbr * (lu ? 2 : 1) * esz, C.d_coef.n) +
-                                more((size_t)inv_elems * esz, C.d_inv.n) + more((size_t)scr_max * esz, C.d_scr.n);
+                                more((size_t)inv_elems * esz, C.d_inv.n) + more((size_t)scr_max * esz, C.d_scr.n) +
+                                more(vec, C.d_flowY.n) + more(vec, C.d_flowZ.n);
             if (need + need / 8 > mfree) {
-                C.forms_off = true;
-                return build_fact_plan(C, fmode, fp32, zc);
+                route.forms = false;
+                *again = true;
+                return PASTIX_GPU_SUCCESS;
             }
         }
         if (C.d_h16.n < (size_t)(2 * C.h16_plane)) PGPU_CHECK(C.d_h16.alloc(2 * C.h16_plane));
@@ -1274,8 +1275,9 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             mapidx_h.swap(mapidx);
             hsbase_h.swap(hsbase);
         } else {
-            C.tma_failed = true;   // (a map the encoder refuses: plan without TMA)
-            return build_fact_plan(C, fmode, fp32, zc);
+            route.tma = false;   // (a map the encoder refuses: plan without TMA)
+            *again = true;
+            return PASTIX_GPU_SUCCESS;
         }
     } else if (C.tma) {
         std::vector<char> src(C.cblknbr, 0);
@@ -1323,8 +1325,9 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
             mapidx_h = mapidx;
             PGPU_CHECK(C.d_split.upload(split, C.stream));
         } else {
-            C.tma_failed = true;
-            return build_fact_plan(C, fmode, fp32, zc);
+            route.tma = false;
+            *again = true;
+            return PASTIX_GPU_SUCCESS;
         }
     }
     if (C.tma) {
@@ -1536,9 +1539,25 @@ static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
     C.plan_fuse = fuse;
     C.plan_esz = (int)esz;
     C.plan_fmode = fmode;
-    C.plan_fact = key;
     C.plan_gemm_flops = gflops;
     C.tc_flops = tcflops;
+    return PASTIX_GPU_SUCCESS;
+}
+
+static int build_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc) {
+    // (set_tuning, set_cblk_priority and structure invalidate the plan: they need no place in the key)
+    const int key = ((fmode * 2 + (fp32 ? 1 : 0)) * 2 + (zc ? 1 : 0)) * 2 + (C.record ? 1 : 0);
+    if (C.plan_fact == key) return PASTIX_GPU_SUCCESS;
+    C.plan_fact = -1;      // (a plan that fails half-way is nobody's,
+    C.fact_done = -1;      // and the factor at hand loses its inverses and solve lists to the new one)
+    invalidate_graph(C);   // the launch lists and workspaces the graph names are rebuilt
+    PlanRoute route;
+    for (bool again = true; again;) {
+        again = false;
+        const int rc = make_fact_plan(C, fmode, fp32, zc, route, &again);
+        if (rc) return rc;
+    }
+    C.plan_fact = key;
     return PASTIX_GPU_SUCCESS;
 }
 

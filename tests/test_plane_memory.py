@@ -95,3 +95,26 @@ def test_a_plan_that_fails_leaves_no_factor():
     s.numfact(A.values)
     assert _check(s, A) > 0
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fact,make", [
+    ("sytrf", lambda: M.diffusion_lognormal(40, 39, 41, 1.0, RNG(2))),
+    ("hetrf", lambda: M.magnetic_laplacian(30, 29, 31, 0.5, RNG(3))),
+], ids=["sytrf", "hetrf"])
+def test_no_room_for_the_planes_lasts_one_plan(fact, make):
+    """LDL and complex planes that do not fit send their updates to the FMA tiles; the next plan, with room
+    again, has them on the tensor cores."""
+    from pastix_b200 import autotune as AT
+    A = make()
+    st = analysis.analyze(A)
+    room = (_takes(A, st, fact) + _takes(A, st, fact, mixed_gemm=0)) // 2
+    s = _solver(A, st, fact)
+    with _only(room):
+        s.numfact(A.values)
+        assert _check(s, A) == 0
+        s.numfact(A.values)
+    AT.set_knob(s, "tc_min_mn", 8192)      # (the default: any knob asks for a new plan)
+    s.numfact(A.values)
+    assert _check(s, A) > 0
+    s.close()
