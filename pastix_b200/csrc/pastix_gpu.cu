@@ -1196,7 +1196,7 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
         auto tall = [&](int c) { return tgemm && C.height[c] > fuse && C.height[c] > C.width[c]; };
         auto needed = [&](int c, int kind) {
             switch (kind) {
-            case TMAP_L: return true;
+            case TMAP_L: return !(zc && ldl) || tall(c);   // (complex LDL updates read L D and the B rows)
             case TMAP_U: return lu || ldl;
             case TMAP_I: return tall(c);
             case TMAP_I2: return lu && tall(c);

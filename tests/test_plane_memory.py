@@ -118,3 +118,35 @@ def test_no_room_for_the_planes_lasts_one_plan(fact, make):
     s.numfact(A.values)
     assert _check(s, A) > 0
     s.close()
+
+
+def _copies(nb, w, m, rng):
+    """nb independent Hermitian systems, each a cblk of w columns with m rows that face a second cblk."""
+    k = w + m
+    v = np.tril(rng.uniform(-1, 1, (nb, k, k)) + 1j * rng.uniform(-1, 1, (nb, k, k)), -1)
+    v[:, np.arange(k), np.arange(k)] = 2.0 * k
+    o = np.arange(nb) * k
+    cblk = [r for i, f in enumerate(o) for r in ([f, f + w - 1, 3 * i, 0], [f + w, f + k - 1, 3 * i + 2, 0])]
+    blok = [r for i, f in enumerate(o) for r in ([f, f + w - 1, 2 * i, 2 * i], [f + w, f + k - 1, 2 * i, 2 * i + 1],
+                                                 [f + w, f + k - 1, 2 * i + 1, 2 * i + 1])]
+    n = nb * k
+    st = dict(n=n, cblktab=np.array(cblk + [[n, n, 3 * nb, 0]], np.int64), bloktab=np.array(blok, np.int64),
+              browtab=np.zeros(nb, np.int64), permtab=np.arange(n), peritab=np.arange(n))
+    r, c = np.tril_indices(k)
+    order = np.lexsort((r, c))
+    r, c = r[order], c[order]
+    colptr = np.concatenate([[0], np.cumsum(np.tile(k - np.arange(k), nb))]).astype(np.int64)
+    A = M.SparseSystem(n, colptr, (o[:, None] + r[None, :]).ravel().astype(np.int64), v[:, r, c].ravel(),
+                       M.PastixHermitian, (n, 1, 1))
+    return A, st
+
+
+@pytest.mark.gpu
+def test_complex_ldl_keeps_no_plane_of_bare_rows():
+    """Its updates read the rows times D and the B rows (two per row); the bare rows are an operand of the tall
+    panels' TRSM only, and these panels are short: three planes of rows, not four."""
+    nb, w, m = 64, 100, 150
+    A, st = _copies(nb, w, m, RNG(5))
+    plane = nb * (w + m) * ((2 * w + 63) // 64 * 64) * 4      # hi and lo halves of every row
+    more = _takes(A, st, "hetrf") - _takes(A, st, "hetrf", mixed_gemm=0)
+    assert 2.5 * plane < more < 3.5 * plane
