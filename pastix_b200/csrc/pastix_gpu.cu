@@ -217,6 +217,7 @@ struct pastix_gpu_s {
     DArr<float> d_hscale;
     DArr<int64_t> d_hoff, d_hsbase;
     int64_t h16_plane = 0;
+    int h16_pitch = 64;       // halves a plane row is padded to (ld16_of)
     // per task its target-row map's base, and
     // the target rows of the tensor-core update tasks (k_task_rowmap)
     DArr<int64_t> d_taux;
@@ -1207,35 +1208,47 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
         auto map_rows = [&](int c, int kind) {
             return (kind == TMAP_I || kind == TMAP_I2 ? C.width[c] : C.height[c]) * (kind >= TMAP_I ? cs : 1);
         };
-        for (int l = 0; l < C.nlevels; l++)
-            for (int q = C.lvl_ptr[l]; q < C.lvl_ptr[l + 1]; q++) {
-                const int c = C.lvl_cblks[q];
-                if (!src[c]) continue;
-                const int w = C.width[c];
-                mapidx[c] = (int)hoff.size();
-                for (int kind = 0; kind < TMAP_KINDS; kind++) {
-                    const bool nd = needed(c, kind);
-                    const int rows = map_rows(c, kind);
-                    hoff.push_back(nd ? hp : -1);
-                    hsbase.push_back(nd ? sp : -1);
-                    if (nd) {
-                        hp += round_up((int64_t)rows * ld16_of(cs * w), 64);
-                        sp += rows;
+        auto layout = [&](int pitch) {
+            C.h16_pitch = pitch;
+            hoff.clear();
+            hsbase.clear();
+            hp = sp = 0;
+            for (int l = 0; l < C.nlevels; l++)
+                for (int q = C.lvl_ptr[l]; q < C.lvl_ptr[l + 1]; q++) {
+                    const int c = C.lvl_cblks[q];
+                    if (!src[c]) continue;
+                    mapidx[c] = (int)hoff.size();
+                    for (int kind = 0; kind < TMAP_KINDS; kind++) {
+                        const bool nd = needed(c, kind);
+                        const int rows = map_rows(c, kind);
+                        hoff.push_back(nd ? hp : -1);
+                        hsbase.push_back(nd ? sp : -1);
+                        if (nd) {
+                            hp += round_up((int64_t)rows * ld16_of(cs * C.width[c], pitch), 64);
+                            sp += rows;
+                        }
                     }
                 }
-            }
-        C.h16_plane = round_up(std::max<int64_t>(hp, 64), 64);
-        if (zc || ldl) {
-            // (complex planes are three times the factor: where they do not fit beside it, FMA tiles)
-            size_t mfree = 0, mtotal = 0;
-            PGPU_CHECK(cudaMemGetInfo(&mfree, &mtotal));
+            C.h16_plane = round_up(std::max<int64_t>(hp, 64), 64);
+        };
+        // whether the planes fit beside everything else a factorization and its solve allocate
+        size_t mfree = 0, mtotal = 0;
+        PGPU_CHECK(cudaMemGetInfo(&mfree, &mtotal));
+        auto fits = [&]() {
             auto more = [](size_t want, size_t have) { return want > have ? want - have : 0; };
             const size_t vec = (size_t)C.n * flow_maxrhs(esz) * esz;   // the dataflow solve's Y, Z
             const size_t need = more(4 * (size_t)C.h16_plane, C.d_h16.n * 2) +
                                 more((size_t)C.coefnbr * (lu ? 2 : 1) * esz, C.d_coef.n) +
                                 more((size_t)inv_elems * esz, C.d_inv.n) + more((size_t)scr_max * esz, C.d_scr.n) +
                                 more(vec, C.d_flowY.n) + more(vec, C.d_flowZ.n);
-            if (need + need / 8 > mfree) {
+            return need + need / 8 <= mfree;
+        };
+        // whole lines where there is room, else packed rows (up to a third smaller; 100^3 takes 1 % longer with
+        // them); the LDL and complex forms, whose planes are two to three times the factor, else go to FMA tiles
+        layout(64);
+        if (!fits()) {
+            layout(8);
+            if ((zc || ldl) && !fits()) {
                 route.forms = false;
                 *again = true;
                 return PASTIX_GPU_SUCCESS;
@@ -1254,7 +1267,8 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
                 for (int kind = 0; kind < TMAP_KINDS; kind++) {
                     const int mi = mapidx[c] + kind;
                     if (hoff[mi] < 0) continue;
-                    if (!encode_h16_map(&maps[mi], C.d_h16.p + hoff[mi], cs * w, map_rows(c, kind), ld16_of(cs * w),
+                    if (!encode_h16_map(&maps[mi], C.d_h16.p + hoff[mi], cs * w, map_rows(c, kind),
+                                        ld16_of(cs * w, C.h16_pitch),
                                         C.h16_plane))
                         C.tma = false;
                     // panels: their off-diagonal rows; inverses: all rows
@@ -1744,7 +1758,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                 k_split_rows_h16<T><<<nsp, 256, 0, s>>>(C.meta, C.d_split.p + C.split_ptr[l], coefL, coefU,
                                                         reinterpret_cast<const T *>(C.d_inv.p), C.d_h16.p,
                                                         C.h16_plane, C.d_hscale.p, C.d_hoff.p, C.d_hsbase.p,
-                                                        C.d_mapidx.p, fm_ldl(fmode) ? 1 : 0,
+                                                        C.d_mapidx.p, C.h16_pitch, fm_ldl(fmode) ? 1 : 0,
                                                         (CPX && fm_conj(fmode)) ? 1 : 0);
                 nl++;
             } else if (C.tma && nsp) {
@@ -1958,7 +1972,7 @@ static int run_factor(pastix_gpu_t &C, int fmode, int *launches, LaunchTimer &tm
                     if (ntr)
                         k_trsm_copyback_h16<T><<<ntr, 256, 0, s>>>(
                             C.meta, C.d_trsm.p + C.trsm_ptr[l], C.d_scroff.p, scr, coefL, coefU, C.d_h16.p,
-                            C.h16_plane, C.d_hscale.p, C.d_hoff.p, C.d_hsbase.p, C.d_mapidx.p,
+                            C.h16_plane, C.d_hscale.p, C.d_hoff.p, C.d_hsbase.p, C.d_mapidx.p, C.h16_pitch,
                             fm_ldl(fmode) ? 1 : 0, (CPX && fm_conj(fmode)) ? 1 : 0);
                     copied = true;
                 }

@@ -703,7 +703,8 @@ __global__ void k_task_rowmap(Meta m, const GemmTask *__restrict__ tasks, const 
 // element in the planes (hoff, rows of ld16 halves, a multiple of 64 that holds
 // the row's floats, so that no 128-byte box row straddles two lines: 80^3 LU
 // 39.1 -> 38.8 ms) and the first row in hscale (hsbase).
-__host__ __device__ inline int ld16_of(int nf) { return (nf + 63) & ~63; }   // whole 128-byte lines: one per box row
+// pitch: 64 halves, whole 128-byte lines, one per box row; 8 (the alignment of a tensor map's rows) where memory is short
+__host__ __device__ inline int ld16_of(int nf, int pitch) { return (nf + pitch - 1) & -pitch; }
 constexpr int H16_MAXW = 400;   // widest cblk (pastix_gpu_structure)
 
 // The pivots of cblk c (LDL: diagonal of its panel) into shared memory.
@@ -722,13 +723,13 @@ __global__ void __launch_bounds__(256) k_split_rows_h16(Meta m, const int4 *__re
                                                         int64_t hplane, float *__restrict__ hscale,
                                                         const int64_t *__restrict__ hoff,
                                                         const int64_t *__restrict__ hsbase,
-                                                        const int *__restrict__ mapidx, int ldl, int cj) {
+                                                        const int *__restrict__ mapidx, int pitch, int ldl, int cj) {
     constexpr bool CX = is_cplx<T>::value;
     __shared__ __align__(16) unsigned char ds_raw[H16_MAXW * sizeof(T)];
     T *ds = reinterpret_cast<T *>(ds_raw);
     const int4 jb = jobs[blockIdx.x];
     const int c = jb.x, r0 = jb.y, kind = jb.z;
-    const int w = m.width[c], ld = m.ld[c], nf = CX ? 2 * w : w, l16 = ld16_of(nf);
+    const int w = m.width[c], ld = m.ld[c], nf = CX ? 2 * w : w, l16 = ld16_of(nf, pitch);
     const bool isinv = kind == TMAP_I || kind == TMAP_I2, upper = kind == TMAP_U || kind == TMAP_BU;
     const int rows = isinv ? w : m.height[c];
     const T *src = isinv ? inv + m.invoff[c] + (kind == TMAP_I2 ? inv_span(w, ld) : 0)
@@ -764,13 +765,13 @@ __global__ void __launch_bounds__(256) k_trsm_copyback_h16(Meta m, const int4 *_
                                                            int64_t hplane, float *__restrict__ hscale,
                                                            const int64_t *__restrict__ hoff,
                                                            const int64_t *__restrict__ hsbase,
-                                                           const int *__restrict__ mapidx, int ldl, int cj) {
+                                                           const int *__restrict__ mapidx, int pitch, int ldl, int cj) {
     constexpr bool CX = is_cplx<T>::value;
     __shared__ __align__(16) unsigned char ds_raw[H16_MAXW * sizeof(T)];
     T *ds = reinterpret_cast<T *>(ds_raw);
     const int4 ch = chunks[blockIdx.x];
     const int c = ch.x, r0 = ch.y;
-    const int w = m.width[c], h = m.height[c], ld = m.ld[c], nf = CX ? 2 * w : w, l16 = ld16_of(nf);
+    const int w = m.width[c], h = m.height[c], ld = m.ld[c], nf = CX ? 2 * w : w, l16 = ld16_of(nf, pitch);
     const int nr = min(32, h - r0);
     const T *src = scr + scroff[c] + (ch.z ? inv_span(h - w, ld) : 0) + (int64_t)(r0 - w) * ld;
     T *dst = (ch.z ? coefU : coefL) + m.coefoff[c] + (int64_t)r0 * ld;

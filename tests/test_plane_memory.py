@@ -150,3 +150,25 @@ def test_complex_ldl_keeps_no_plane_of_bare_rows():
     plane = nb * (w + m) * ((2 * w + 63) // 64 * 64) * 4      # hi and lo halves of every row
     more = _takes(A, st, "hetrf") - _takes(A, st, "hetrf", mixed_gemm=0)
     assert 2.5 * plane < more < 3.5 * plane
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fact,make", [
+    ("potrf", lambda: M.diffusion_lognormal(50, 49, 51, 1.0, RNG(2))),
+    ("getrf", lambda: M.convdiff_upwind(50, 49, 51, 10.0)),
+], ids=["potrf", "getrf"])
+def test_planes_are_packed_where_whole_lines_do_not_fit(fact, make):
+    """What fitted with rows padded to 8 halves still does."""
+    A = make()
+    st = analysis.analyze(A)
+    w = st["cblktab"][:-1, 1] - st["cblktab"][:-1, 0] + 1
+    rows = np.concatenate([[0], np.cumsum(st["bloktab"][:, 1] - st["bloktab"][:, 0] + 1)])
+    h = rows[st["cblktab"][1:, 2]] - rows[st["cblktab"][:-1, 2]]
+    src = (w >= 64) & (h >= w + 128)                         # (a lower bound: sources of tensor-core updates)
+    pad = 4 * int((h * ((w + 63) // 64 * 64 - (w + 7) // 8 * 8))[src].sum()) * (2 if fact == "getrf" else 1)
+    assert pad > 24 * 2 ** 20
+    s = _solver(A, st, fact)
+    with _only(_takes(A, st, fact) - pad // 2):
+        s.numfact(A.values)
+        assert _check(s, A) > 0
+    s.close()
