@@ -692,12 +692,14 @@ static int fact_mode_of(int fact, bool zc) {
 // (0: none at all), narrower ones where the level has few of them: the one-CTA
 // form (k_panel_factor) finishes a 64-column panel in about the time its block
 // rows take to hand over one tile each, and leaves the other SMs to the rest
-// of a level of thousands; below four such blocks per SM the chain counts
-// (20^3 FP64, levels of 1-16 blocks: 1.33 -> 0.52 ms of panels).
-const int PR_FEW = 592;
-static bool rows_panel(const pastix_gpu_t &C, int w, size_t esz, bool lu, int nlvl) {
+// of a level of thousands; up to four such blocks per SM (`few`) the chain
+// counts (20^3 FP64, levels of 1-16 blocks: 1.33 -> 0.52 ms of panels).
+// Blocks whose row of tiles does not fit in shared memory (LU in FP64 and
+// complex64 and the other complex128 forms above 320 columns, complex128 LU
+// above 128) stay with the one-CTA form.
+static bool rows_panel(const pastix_gpu_t &C, int w, size_t esz, bool lu, int nlvl, int few) {
     const int64_t wmin = C.tune[PGPU_TUNE_WIDE_PANEL];
-    return wmin > 0 && w > PB && (w >= wmin || nlvl <= PR_FEW) && pr_slots(w, esz, lu, WP_SMEM_LIMIT) > 0;
+    return wmin > 0 && w > PB && (w >= wmin || nlvl <= few) && pr_slots(w, esz, lu, WP_SMEM_LIMIT) > 0;
 }
 
 // Forget the captured factorization graph (its nodes name the plan's and the
@@ -924,6 +926,8 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
     const int fuse = tgemm ? std::min((int)C.tune[PGPU_TUNE_TRSM_GEMM_ROWS], fuse_rows_for(lu, esz))
                            : fuse_rows_for(lu, esz);
     const bool tc_trsm = tgemm && ((fp32 && tc_enabled(C) && (!zc || h16_forms)) || use_dmma);
+    int nsm_plan = 148;
+    PGPU_CHECK(cudaDeviceGetAttribute(&nsm_plan, cudaDevAttrMultiProcessorCount, C.device));
     std::vector<int2> invjobs;
     std::vector<int4> ttiles, tttiles;
     int64_t inv_elems = 0, scr_max = 0;
@@ -1007,7 +1011,7 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
             const int c = C.lvl_cblks[q];
             const int w = C.width[c], h = C.height[c];
             const int rows = (h <= fuse) ? h : w;
-            const bool by_rows = rows_panel(C, w, esz, lu, nlvl);
+            const bool by_rows = rows_panel(C, w, esz, lu, nlvl, 4 * nsm_plan);
             const int nt = cdiv(w, PB), pr_cnt = C.pr_counters, pr_tile = prscr;
             // the jobs that invert the diagonal block (after the panel's own)
             auto inverse_jobs = [&](int sides) {
@@ -1243,8 +1247,9 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
                                 more(vec, C.d_flowY.n) + more(vec, C.d_flowZ.n);
             return need + need / 8 <= mfree;
         };
-        // whole lines where there is room, else packed rows (up to a third smaller; 100^3 takes 1 % longer with
-        // them); the LDL and complex forms, whose planes are two to three times the factor, else go to FMA tiles
+        // whole lines where there is room, else packed rows (up to a third smaller; 80^3 LU 38.8 -> 39.1 ms a call,
+        // 60^3 complex LDL^h 21.7 -> 21.9); the LDL and complex forms, whose planes are two to three times the
+        // factor, else go to FMA tiles
         layout(64);
         if (!fits()) {
             layout(8);
@@ -1350,8 +1355,6 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
             // share their B tile in the TMA kernel: one entry {task, tm, tn, 1}
             // (a launch with fewer tiles than two per SM keeps them single: pairs
             // would leave SMs idle)
-            int nsm_plan = 148;
-            PGPU_CHECK(cudaDeviceGetAttribute(&nsm_plan, cudaDevAttrMultiProcessorCount, C.device));
             const int64_t pmin = C.tune[PGPU_TUNE_TC_PAIR_MIN] >= 0 ? C.tune[PGPU_TUNE_TC_PAIR_MIN] : 2 * nsm_plan;
             auto pair_range = [pmin](const std::vector<int4> &in, int b, int e, std::vector<int4> &out) {
                 if (e - b < pmin) {
