@@ -160,56 +160,6 @@ __device__ __forceinline__ void warp_factor_tile(T *tile, int nb, typename real_
     }
 }
 
-// Shared-memory form of the same factorization (the tile stays in shared
-// memory, lane 0 evaluates the pivots): for kernels whose register budget
-// cannot hold a row of 8-byte elements next to their other live values.
-template <typename T, int MODE>
-__device__ __forceinline__ void warp_factor_tile_smem(T *tile, int nb, typename real_of<T>::type crit, int &npiv,
-                                                      int &nneg, int &nbad) {
-    typedef typename real_of<T>::type R;
-    constexpr bool CJ = fm_conj(MODE);
-    const int lane = threadIdx.x & 31;
-    for (int k = 0; k < nb; k++) {
-        if (lane == 0) {
-            T a = tile[k * PBL + k];
-            if (!finite_v(a)) nbad++;
-            a = static_pivot<T, MODE>(a, crit, npiv);
-            if (MODE == FM_POTRF) {
-                if (real_v(a) < R(0)) nneg++;
-                a = sqrt_v(a);
-            }
-            tile[k * PBL + k] = a;
-        }
-        __syncwarp();
-        const T dk = tile[k * PBL + k];
-        const T inv = T(1) / (MODE == FM_POTRF ? cj<CJ>(dk) : dk);
-        if (lane > k && lane < nb) tile[lane * PBL + k] = tile[lane * PBL + k] * inv;
-        __syncwarp();
-        if (lane > k && lane < nb) {
-            const T lik = tile[lane * PBL + k];
-            // 8 entries per batch: their loads are issued before the stores
-            // (the compiler cannot reorder shared-memory loads past stores)
-            const int jend = (MODE == FM_GETRF) ? nb - 1 : lane;
-            const T f = (MODE == FM_GETRF || MODE == FM_POTRF) ? lik : lik * (MODE == FM_HETRF ? T(real_v(dk)) : dk);
-            for (int j0 = k + 1; j0 <= jend; j0 += 8) {
-                T src[8], cur[8];
-#pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    const int j = min(j0 + u, jend);
-                    src[u] = (MODE == FM_GETRF) ? tile[k * PBL + j] : cj<CJ>(tile[j * PBL + k]);
-                    cur[u] = tile[lane * PBL + j];
-                }
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (j0 + u <= jend) tile[lane * PBL + j0 + u] = cur[u] - f * src[u];
-            }
-            // LDL^h takes the real part of d_k (zher)
-            if (MODE == FM_HETRF) tile[lane * PBL + lane] = T(real_v(tile[lane * PBL + lane]));
-        }
-        __syncwarp();
-    }
-}
-
 // Row solves against the factorized tile (x: nb values of one row, in place).
 //   lower_t: x op(L)^t = a, L = lower of the tile (unit when `unit`), op =
 //            conj when CJ -- POTRF rows, LU U^t rows, LDL rows (unit);
