@@ -342,6 +342,13 @@ PASTIX_GPU_API int pastix_gpu_coeftab( pastix_gpu_t *ctx, void *L, void *U );
 PASTIX_GPU_API int pastix_gpu_stats( pastix_gpu_t *ctx, double *stats );
 
 /*
+ * Tile counts of the last numfact's plan: counts[0] tensor-core update tiles,
+ * counts[1] those that sum the updates of several source cblks (single
+ * precision), counts[2] of these the pairs of 128-row tiles.  (3 int64_t)
+ */
+PASTIX_GPU_API int pastix_gpu_plan_counts( pastix_gpu_t *ctx, int64_t *counts );
+
+/*
  * Host analysis for a matrix on an nx x ny x nz grid (vertex x + nx*(y + ny*z)):
  * the reference's grid nested dissection (pastixOrderGrid,
  * order/order_grids.c:303) with the personal-ordering analysis that follows

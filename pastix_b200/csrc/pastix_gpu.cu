@@ -151,6 +151,7 @@ struct pastix_gpu_s {
     std::vector<int> ps_ptr;   // cblks of at most 32 columns: one warp each (k_panel_small)
     DArr<int2> d_sjobs;
     DArr<int4> d_tiles, d_tctiles, d_trsm;
+    int64_t plan_counts[3] = {0, 0, 0};   // tensor-core update tiles; of several sources; of these, pairs
     double tc_flops = 0;   // update-GEMM flops on the tensor-core path
     DArr<GemmTask> d_tasks;
     std::vector<int> solve_ptr;
@@ -1433,6 +1434,8 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
     PGPU_CHECK(C.d_tctiles.upload(tctiles, s));
     PGPU_CHECK(C.d_trsm.upload(trsm, s));
     PGPU_CHECK(C.d_tasks.upload(tasks, s));
+    C.plan_counts[0] = (int64_t)tctiles.size();
+    C.plan_counts[1] = C.plan_counts[2] = 0;
     if (C.tma || use_dmma) {
         // tensor-core tasks: target-row maps (built on the device)
         std::vector<int64_t> taux(tasks.size(), 0);
@@ -1453,7 +1456,7 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
         if (C.tma) {
             // the segments of a batch's tasks (of a TRSM task), contiguous
             std::vector<TcSeg> segs;
-            std::vector<int> seg0(tasks.size(), -1), nseg(tasks.size(), 0);
+            std::vector<int> seg0(tasks.size(), -1), nseg(tasks.size(), 0), nsrc(tasks.size(), 0);
             // k-blocks of a segment (k_gemm_scatter_tc_tma): all of a source in real LL^t and LU, whose sums are as
             // close as they always were; 64 columns in the LDL and complex forms, whose sums the FMA tiles rounded
             // to nearest.  Error of the factor, whole depth -> 64 columns (FMA tiles), and of the call's time:
@@ -1488,6 +1491,7 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
                 seg0[lead] = (int)segs.size();
                 for (int id : ids) add_seg(id);
                 nseg[lead] = (int)segs.size() - seg0[lead];
+                nsrc[lead] = (int)ids.size();
             };
             for (const auto &bt : batches) add_tile(bt[0], bt);
             for (const int4 &t : tttiles)
@@ -1524,7 +1528,11 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
                 return d;
             };
             std::vector<TcDesc> dtc(tctiles.size()), dtt(tttiles.size());
-            for (size_t i = 0; i < tctiles.size(); i++) dtc[i] = make_desc(tctiles[i]);
+            for (size_t i = 0; i < tctiles.size(); i++) {
+                dtc[i] = make_desc(tctiles[i]);
+                C.plan_counts[1] += nsrc[tctiles[i].x] > 1;
+                C.plan_counts[2] += nsrc[tctiles[i].x] > 1 && dtc[i].pair;
+            }
             for (size_t i = 0; i < tttiles.size(); i++) dtt[i] = make_desc(tttiles[i]);
             PGPU_CHECK(C.d_tcdesc.upload(dtc, s));
             PGPU_CHECK(C.d_ttdesc.upload(dtt, s));
@@ -3580,6 +3588,12 @@ extern "C" int pastix_gpu_phase_log(pastix_gpu_t *ctx, int64_t *count, int64_t *
     std::memcpy(info, ctx->phase_info.data(), 3 * k * sizeof(int64_t));
     std::memcpy(times, ctx->phase_times.data(), 2 * k * sizeof(double));
     *count = k;
+    return PASTIX_GPU_SUCCESS;
+}
+
+extern "C" int pastix_gpu_plan_counts(pastix_gpu_t *ctx, int64_t *counts) {
+    if (!ctx || !counts || ctx->plan_fact < 0) return PASTIX_GPU_ERR_BADPARAMETER;
+    std::memcpy(counts, ctx->plan_counts, sizeof(ctx->plan_counts));
     return PASTIX_GPU_SUCCESS;
 }
 

@@ -31,7 +31,7 @@ ERRORS = {1: "PASTIX_ERR_UNKNOWN", 2: "PASTIX_ERR_ALLOC", 3: "PASTIX_ERR_NOTIMPL
 EXPORTS = ["pastix_gpu_init", "pastix_gpu_structure", "pastix_gpu_spm", "pastix_gpu_numfact",
            "pastix_gpu_solve", "pastix_gpu_refine", "pastix_gpu_solve_and_refine",
            "pastix_gpu_get_params", "pastix_gpu_set_iparm", "pastix_gpu_set_dparm",
-           "pastix_gpu_coeftab", "pastix_gpu_stats", "pastix_gpu_finalize"]
+           "pastix_gpu_coeftab", "pastix_gpu_stats", "pastix_gpu_plan_counts", "pastix_gpu_finalize"]
 
 
 class PastixGpuError(RuntimeError):
@@ -63,6 +63,7 @@ def load():
         L.pastix_gpu_set_dparm.argtypes = [P, I, D]
         L.pastix_gpu_coeftab.argtypes = [P, P, P]
         L.pastix_gpu_stats.argtypes = [P, P]
+        L.pastix_gpu_plan_counts.argtypes = [P, P]
         L.pastix_gpu_set_segments.argtypes = [P, I64, P]
         L.pastix_gpu_finalize.argtypes = [C.POINTER(P)]
         L.pastix_gpu_finalize.restype = None
@@ -133,6 +134,13 @@ class Solver:
                 "refine_ms", "gemm_ms", "gemm_launches", "diag_ms", "trsm_ms", "gemm_flops", "tc_ms",
                 "tc_flops", "tc_timeouts", "graph_replayed", "spm_ms"]
         return dict(zip(keys, s.tolist()))
+
+    def plan_counts(self):
+        """Tensor-core update tiles of the last numfact's plan, those that sum several source cblks, and
+        the pairs of 128-row tiles among these."""
+        c = np.zeros(3, np.int64)
+        _check("pastix_gpu_plan_counts", load().pastix_gpu_plan_counts(self._h, _p(c)))
+        return tuple(int(v) for v in c)
 
     def phase_log(self):
         """Timeline of the last directly launched numfact: a list of

@@ -32,9 +32,12 @@ def test_dataflow_solve_any_number_of_right_hand_sides(fact, make, mixed, nrhs):
     b[:, nrhs // 2] *= 1e6      # (a column of another scale: no mixing between columns)
     x[:, nrhs // 2] *= 1e6
     got = s.solve(b)
+    launches = s.stats()["solve_launches"]
     AT.set_knob(s, "solve_flow", 0)
     s.numfact(A.values)
     ref = s.solve(b)
+    # the runs of levels went through the dataflow: a launch a pass each way instead of four a level
+    assert launches < s.stats()["solve_launches"]
     err, base = (np.linalg.norm(v - x, axis=0) / np.linalg.norm(x, axis=0) for v in (got, ref))
     # both are the same factor's solves: rounding of another order of the same sums
     u = 2.0 ** (-24 if mixed else -53)

@@ -92,14 +92,18 @@ def test_tensor_core_forms_match_restatement(fact, make, mixed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("fact,make", [
-    ("potrf", lambda: M.diffusion_lognormal(40, 37, 39, 1.0, RNG(8))),
-    ("getrf", lambda: M.convdiff_upwind(36, 35, 37, 10.0)),
-    ("hetrf", lambda: M.magnetic_laplacian(33, 34, 32, 0.5, RNG(9))),
-], ids=["potrf", "getrf", "hetrf"])
-def test_fan_in_over_separator_chains(fact, make):
+@pytest.mark.parametrize("fact,make,mode", [
+    ("potrf", lambda: M.diffusion_lognormal(40, 37, 39, 1.0, RNG(8)), 3),
+    ("sytrf", lambda: M.diffusion_lognormal(40, 37, 39, 1.0, RNG(8)), 3),
+    ("getrf", lambda: M.convdiff_upwind(36, 35, 37, 10.0), 3),
+    ("hetrf", lambda: M.magnetic_laplacian(33, 34, 32, 0.5, RNG(9)), 3),
+    ("potrf", lambda: M.diffusion_lognormal(40, 37, 39, 1.0, RNG(8)), 2),
+    ("getrf", lambda: M.convdiff_upwind(36, 35, 37, 10.0), 2),
+], ids=["potrf", "sytrf", "getrf", "hetrf", "potrf_3xtf32", "getrf_3xtf32"])
+def test_fan_in_over_separator_chains(fact, make, mode):
     """Separators wide enough for chains of several cblks, whose deferred updates are summed before they
-    are scattered: the factor agrees with the FMA tiles', which scatter every source on its own."""
+    are scattered, in single tiles and in pairs (mode 3: 3xFP16, 2: 3xTF32, without row scales): the factor
+    agrees with the FMA tiles', which scatter every source on its own."""
     from pastix_b200 import autotune as AT
     from pastix_b200 import gpu as G
     A = make()
@@ -109,8 +113,12 @@ def test_fan_in_over_separator_chains(fact, make):
     s.set_iparm(G.IPARM_MIXED, 1)
     s.set_structure(st)
     s.set_spm(A)
+    AT.set_knob(s, "mixed_gemm", mode)
+    AT.set_knob(s, "tc_pair_min", 0)
     s.numfact(A.values)
     assert s.stats()["tc_flops"] > 0.8 * s.stats()["gemm_flops"]
+    tiles, several, pairs = s.plan_counts()
+    assert tiles > several > pairs > 0
     L, U = s.coeftab()
     AT.set_knob(s, "mixed_gemm", 0)
     s.numfact(A.values)
