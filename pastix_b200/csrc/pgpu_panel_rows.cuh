@@ -8,7 +8,8 @@
 // row in shared memory from the first load to the last store.  At step k it
 //   1. waits for row k's diagonal tile (its inverse is published in `scr`),
 //   2. X_ik = A_ik op(L_kk)^{-1} (LU: U_kk^{-1}) as a product with that inverse,
-//      stored into the panel and published,
+//      corrected once by its residual (solve_tile), stored into the panel and
+//      published,
 //   3. A_ij -= X_ik op(L_jk)^t for k < j <= i with the rows' X_jk read through
 //      L2 as they are published (LU: U_kj^t in place of L_jk; the CTA holds
 //      column i of U, transposed, beside row i of L, and updates it alike),
@@ -22,13 +23,13 @@
 // launch is resident makes progress.  All waits are bounded (Status::panel_timeout).
 //
 // What bounds it: the chain of w / 32 steps, each one L2 round trip (poll and
-// tile), two 32^3 products, and the 32-column elimination of the tile on one
+// tiles), four 32^3 products, and the 32-column elimination of the tile on one
 // warp; the other rows' updates run beside it.  With one CTA for the whole
 // block the rank-32 updates of one SM bounded it.  Block and inverse of a
 // root-chain cblk of ~320 columns on one B200, from 512-thread CTA + inverse
-// kernel to this: FP32 LL^t 300 -> 110 us, FP64 LL^t 750 -> 165, FP32 LU 380 ->
-// 145, complex64 LDL^h 1150 -> 290; 20^3 FP64 factor + solve 2.53 -> 1.54 ms,
-// 37x45x51 FP64 LU 20.7 -> 11.2, 41x33x47 complex128 LDL^h 38.5 -> 18.8.
+// kernel to this (without the products' correction): FP32 LL^t 300 -> 110 us,
+// FP64 LL^t 750 -> 165, FP32 LU 380 -> 145, complex64 LDL^h 1150 -> 290; the
+// 20^3 FP64 factor + solve 2.53 -> 1.54 ms (with it some 0.07 more).
 #pragma once
 
 #include "pgpu_common.cuh"
@@ -58,8 +59,8 @@ inline int pr_slots(int w, size_t esz, bool lu, size_t limit) {
 inline size_t pr_smem_bytes(int w, size_t esz, bool lu, int slots) {
     return (size_t)(pr_row_tiles(w, lu) + 1 + slots) * PB * (PB + 16 / esz) * esz;
 }
-// Published per diagonal tile: T = L^{-1} (32 x 32), LU: V = (U^t)^{-1}, and 1/d.
-__host__ __device__ constexpr int pr_scr_tile(bool lu) { return (lu ? 2 : 1) * PB * PB + PB; }
+// Published per diagonal tile: T = L^{-1} and L (32 x 32 each), LU: V = (U^t)^{-1} and U^t, and 1/d.
+__host__ __device__ constexpr int pr_scr_tile(bool lu) { return (lu ? 4 : 2) * PB * PB + PB; }
 
 // Jobs {cblk, block row (inverse: column block) | kind << 16, counter of row 0,
 // scratch tile of row 0}.
@@ -319,6 +320,61 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
         }
     };
     auto failed = [&]() { return *(volatile int *)&fail_s != 0; };
+    // x = M op(Ti)^t, then once x += (M - x op(Lt)^t) op(Ti)^t, and with TWO y from N alike (x, y: this thread's
+    // 2 x 2 entries; M and N are overwritten): the product with an inverse alone leaves a residual larger by the
+    // tile's condition than a substitution's, the corrected one does not.  (Solves of shifted, indefinite grids of
+    // some 9000 unknowns with the factor, error without and with: FP64 LDL^t 1.7e-11 -> 8.4e-12, by substitution
+    // 8.0e-12; single precision 1.7e-2 -> 7.5e-3.  It costs 1 to 5 % of a call, the most where the panel chain
+    // is the longest part: 60^3 complex LDL^h 23.0 -> 24.2 ms.)
+    auto solve_tile = [&](auto cb, auto two, T *M, const T *Ti, const T *Lt, T (&x)[2][2], T *N, const T *Ni,
+                          const T *Nt, T (&y)[2][2]) {
+        constexpr bool CB = decltype(cb)::value, TWO = decltype(two)::value;
+        auto own = [&](T *t, int p, int q) -> T & { return t[(y16 + 16 * p) * P + x16 + 16 * q]; };
+        T m[2][2], n[2][2], z[2][2];
+        auto put = [&](const T (&u)[2][2], const T (&v)[2][2]) {
+            __syncthreads();
+#pragma unroll
+            for (int p = 0; p < 2; p++)
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    own(M, p, q) = u[p][q];
+                    if (TWO) own(N, p, q) = v[p][q];
+                }
+            __syncthreads();
+        };
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                m[p][q] = own(M, p, q);
+                if (TWO) n[p][q] = own(N, p, q);
+            }
+        pr_zero(x);
+        pr_mm<2, 16, CB>(M, Ti, y16, x16, x);
+        if (TWO) {
+            pr_zero(y);
+            pr_mm<2, 16, false>(N, Ni, y16, x16, y);
+        }
+        put(x, y);
+        auto residual = [&](T (&r)[2][2]) {
+#pragma unroll
+            for (int p = 0; p < 2; p++)
+#pragma unroll
+                for (int q = 0; q < 2; q++) r[p][q] -= z[p][q];
+        };
+        pr_zero(z);
+        pr_mm<2, 16, CB>(M, Lt, y16, x16, z);
+        residual(m);
+        if (TWO) {
+            pr_zero(z);
+            pr_mm<2, 16, false>(N, Nt, y16, x16, z);
+            residual(n);
+        }
+        put(m, n);
+        pr_mm<2, 16, CB>(M, Ti, y16, x16, x);
+        if (TWO) pr_mm<2, 16, false>(N, Ni, y16, x16, y);
+        __syncthreads();
+    };
 
     if (kind == PR_ROW) {
         const bool diag = i < nt;
@@ -342,18 +398,17 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
             __syncthreads();
             if (failed()) break;
             const T *sk = sc + (int64_t)k * SCR;
-            load_scr(LU ? sk + PB * PB : sk, S);
-            if (LU) load_scr(sk, S + TILE);
-            if (LDL && tid < PB) rsm[tid] = ldcg_s(sk + PB * PB + tid);
+            load_scr(LU ? sk + PB * PB : sk, S);                      // T (LU: V)
+            load_scr(sk + (LU ? 3 : 1) * PB * PB, S + TILE);          // L (LU: U^t)
+            if (LU) {
+                load_scr(sk, S + 2 * TILE);
+                load_scr(sk + 2 * PB * PB, S + 3 * TILE);
+            }
+            if (LDL && tid < PB) rsm[tid] = ldcg_s(sk + 2 * PB * PB + tid);
             __syncthreads();
             T x[2][2], y[2][2];
-            pr_zero(x);
-            pr_mm<2, 16, CJ>(Q, S, y16, x16, x);
-            if (LU) {
-                pr_zero(y);
-                pr_mm<2, 16, false>(V, S + TILE, y16, x16, y);
-            }
-            __syncthreads();
+            solve_tile(std::integral_constant<bool, CJ>{}, std::integral_constant<bool, LU>{}, Q, S, S + TILE, x, V,
+                       S + 2 * TILE, S + 3 * TILE, y);
 #pragma unroll
             for (int p = 0; p < 2; p++)
 #pragma unroll
@@ -451,9 +506,16 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
                 T t = To[r * P + q];
                 if (MODE == FM_POTRF && r < nr) t = t * (T(1) / sqs[r]);
                 so[e] = t;
-                if (LU) so[PB * PB + e] = Vo[r * P + q];
+                const bool in = r < nr && q <= r;
+                T l = !in ? T(0) : q == r ? (MODE == FM_POTRF ? sqs[r] : T(1)) : Lc[q * PB + r - q - 1];
+                if (MODE == FM_POTRF && in && q < r) l = l * sqs[q];
+                so[(LU ? 2 : 1) * PB * PB + e] = l;
+                if (LU) {
+                    so[PB * PB + e] = Vo[r * P + q];
+                    so[3 * PB * PB + e] = !in ? T(0) : q == r ? dsm[r] : Ub[q * PB + r - q - 1];
+                }
             }
-            if (tid < PB) so[(LU ? 2 : 1) * PB * PB + tid] = tid < nr ? rsm[tid] : T(0);
+            if (tid < PB) so[(LU ? 4 : 2) * PB * PB + tid] = tid < nr ? rsm[tid] : T(0);
             __syncthreads();
             if (tid == 0) {
                 __threadfence();
@@ -483,7 +545,7 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
             __syncthreads();
             if (failed()) break;
             const T *sj = sc + (int64_t)j * SCR;
-            if (LDL && tid < PB) rsm[tid] = ldcg_s(sj + PB * PB + tid);
+            if (LDL && tid < PB) rsm[tid] = ldcg_s(sj + 2 * PB * PB + tid);
             load_scr(sj + vo, Tt);
             if (j == i) {
                 __syncthreads();
@@ -515,11 +577,11 @@ __global__ void __launch_bounds__(PR_THREADS, sizeof(T) <= 8 ? 2 : 1) k_panel_ro
                     for (int g = 1; g < slots; g++) s += S[g * TILE + o];
                     X[o] = s;
                 }
+                __syncthreads();                        // (the slots are free: L or U^t of tile j into the first)
+                load_scr(sj + vo + (LU ? 2 : 1) * PB * PB, S);
                 __syncthreads();
                 T x[2][2];
-                pr_zero(x);
-                pr_mm<2, 16, false>(X, Tt, y16, x16, x);
-                __syncthreads();
+                solve_tile(std::false_type{}, std::false_type{}, X, Tt, S, x, X, Tt, S, x);
 #pragma unroll
                 for (int p = 0; p < 2; p++)
 #pragma unroll

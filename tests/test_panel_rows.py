@@ -99,3 +99,55 @@ def test_negative_pivot_is_refused(w, col):
     with pytest.raises(G.PastixGpuError):
         s.numfact(A.values)
     s.close()
+
+
+def _growing(fact, w, m, g, rng):
+    """A = L L^t (LU: L U) whose first 32-column diagonal tile, -g below its diagonal, has an inverse of
+    some (1 + g)^31."""
+    n = w + m
+
+    def lower():
+        v = np.tril(rng.uniform(-1, 1, (n, n)) / 32, -1)
+        v[:32, :32] = np.tril(-g * np.ones((32, 32)), -1)
+        v[:, w:] = 0
+        v[np.arange(n), np.arange(n)] = 1
+        return v
+    L = lower()
+    R = lower().T if fact == "getrf" else L.T
+    v = L @ R
+    v[np.arange(w, n), np.arange(w, n)] += 2.0 * n
+    A = sp.csc_matrix(v if fact == "getrf" else np.tril(v))
+    mtx = M.PastixGeneral if fact == "getrf" else M.PastixSymmetric
+    return v, M.SparseSystem(n, A.indptr.astype(np.int64), A.indices.astype(np.int64), A.data, mtx, (n, 1, 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fact,mixed,w,m", [
+    (f, x, w, m) for f in ("potrf", "sytrf", "getrf") for x in (False, True)
+    for w, m in ([(50, 40), (64, 30)] if f == "getrf" and not x else [(64, 40), (96, 100), (130, 70)])])
+def test_block_rows_solve_as_a_substitution_does(fact, mixed, w, m):
+    """The rows X of the panel leave the residual of a substitution, |A - X U| <= k u |X| |U| (k terms a sum, and
+    a few for the tile's factor), also where the tile's inverse is large: a product with the inverse alone leaves
+    one larger by up to its condition (in single
+    precision a smaller one, the matrix has to stay definite).  Panels that the kernel solves itself: at most 256
+    rows, FP64 LU 96."""
+    v, A = _growing(fact, w, m, 0.2 if mixed else 0.4, np.random.default_rng(w))
+    v = v.astype(np.float32) if mixed else v
+    st = _structure(w, m)
+    s = _solver(A, st, fact, mixed)
+    s.numfact(A.values)
+    L, U = s.coeftab()
+    s.close()
+    lay = NP.Layout(st["cblktab"], st["bloktab"])
+    P = lay.panel(L, 0).astype(np.float64)
+    D, X = P[:w], P[w:]
+    if fact == "getrf":
+        sides = [(v[w:, :w], X, np.triu(D)), (v[:w, w:].T, lay.panel(U, 0).astype(np.float64)[w:],
+                                              (np.tril(D, -1) + np.eye(w)).T)]
+    elif fact == "sytrf":
+        sides = [(v[w:, :w], X, np.diag(np.diag(D)) @ (np.tril(D, -1) + np.eye(w)).T)]
+    else:
+        sides = [(v[w:, :w], X, np.tril(D).T)]
+    u = 2.0 ** (-24 if mixed else -53)
+    for B, X, T in sides:
+        assert np.abs(B - X @ T).max() <= 4 * w * u * (np.abs(X) @ np.abs(T)).max()
