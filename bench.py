@@ -164,11 +164,9 @@ def factor_nnz(st):
 
 
 # DRAM bytes of the tensor-core update kernel over one factorization of the
-# 100^3 lognormal diffusion problem (LL^t, 3xFP16), from a one-pass ncu capture
-# of every launch of a numfact.  The capture in
-# profiles/k_gemm_scatter_tc_tma_c2_dram.md is of the kernel without the fan-in,
-# which writes fewer partial sums: None until the present kernel is captured.
-TC_DRAM_BYTES_100CUBE = None
+# 100^3 lognormal diffusion problem (LL^t, 3xFP16): one-pass ncu capture of all
+# 228 launches of a numfact (profiles/k_gemm_scatter_tc_tma_c2_dram.md).
+TC_DRAM_BYTES_100CUBE = {"read": 55200381696, "write": 13675170560, "launches": 228}
 
 
 def measured_peaks():
@@ -584,11 +582,10 @@ def main():
                      "frac": tc_ach / bf16_peak if (bf16_peak and tc_ach) else None,
                      # DRAM bytes per step of the kernel (ncu capture of this workload; other
                      # configurations were not captured)
-                     "traffic": (TC_DRAM_BYTES_100CUBE["read"] + TC_DRAM_BYTES_100CUBE["write"])
-                                if cfg == 2 and TC_DRAM_BYTES_100CUBE else None,
+                     "traffic": (TC_DRAM_BYTES_100CUBE["read"] + TC_DRAM_BYTES_100CUBE["write"]) if cfg == 2 else None,
                      "traffic_rate_gbs": ((TC_DRAM_BYTES_100CUBE["read"] + TC_DRAM_BYTES_100CUBE["write"]) /
                                           (mixed["tc_ms_per_step"] * 1e-3) / 1e9)
-                                         if (cfg == 2 and TC_DRAM_BYTES_100CUBE and mixed["tc_ms_per_step"]) else None,
+                                         if (cfg == 2 and mixed["tc_ms_per_step"]) else None,
                      "peak_source": "dense BF16/FP16 tensor rate, %s (%s)" % (
                          mp["source"], "MEASURED_PEAKS.json" if mp["source"] == "measured" else
                          "no MEASURED_PEAKS.json: the earlier measurement on this pool"),

@@ -327,7 +327,7 @@ PASTIX_GPU_API int pastix_gpu_coeftab( pastix_gpu_t *ctx, void *L, void *U );
  *   stats[8] diagonal-factorization ms, stats[9] panel-TRSM ms inside numfact
  *   stats[10] algorithmic flops of the update GEMMs (sum of 2 M N K)
  *   stats[11] ms of the tensor-core update-GEMM launches (part of stats[6]): tcgen05
- *             for single precision, DMMA for real FP64
+ *             for single precision, DMMA for FP64
  *   stats[12] algorithmic flops of the GEMM tasks that ran on the tensor cores
  *   stats[13] tensor-core tiles whose bounded MMA wait timed out (0 when healthy)
  *   stats[14] 1 when the factorization replayed a captured CUDA graph
