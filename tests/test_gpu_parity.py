@@ -377,8 +377,8 @@ WIDE_CASES = [
 @pytest.mark.parametrize("fact,make,mixed", WIDE_CASES,
                          ids=["potrf_d", "potrf_s", "getrf_d", "getrf_s", "sytrf_d", "sytrf_s", "hetrf_c", "potrf_c"])
 def test_wide_panel_kernel_matches_narrow(fact, make, mixed):
-    """Diagonal blocks of 128 columns and more go to the left-looking
-    512-thread kernel; with it switched off (PGPU_TUNE_WIDE_PANEL = 0) the
+    """Diagonal blocks of 128 columns and more go to the kernel of one CTA
+    per 32-row block row; with it switched off (PGPU_TUNE_WIDE_PANEL = 0) the
     right-looking panel kernel factorizes them.  Both factors agree to the
     rounding of their different summation orders."""
     from pastix_b200 import autotune as AT
