@@ -3526,7 +3526,8 @@ extern "C" int pastix_gpu_task_times(pastix_gpu_t *ctx, int64_t *count, int64_t 
 static int task_records_impl(pastix_gpu_t *ctx, int64_t *count, int64_t *info, double *ns, int64_t *times) {
     if (!ctx || !count) return PASTIX_GPU_ERR_BADPARAMETER;
     auto &C = *ctx;
-    if (C.fact_done < 0 || !C.record || C.plan_fact < 0) return PASTIX_GPU_ERR_BADPARAMETER;
+    // (the last numfact recorded: the lowest bit of the plan's key)
+    if (C.fact_done < 0 || !C.record || C.plan_fact < 0 || !(C.plan_fact & 1)) return PASTIX_GPU_ERR_BADPARAMETER;
     const int64_t cnt[4] = {C.cblknbr, (int64_t)C.h_trsm.size(), (int64_t)C.h_tiles.size(),
                             (int64_t)C.h_tctiles.size()};
     const int64_t total = cnt[0] + cnt[1] + cnt[2] + cnt[3];

@@ -26,6 +26,9 @@ def test_recording_gets_a_plan_of_its_own(fact, mixed):
     err = []
     for on in (False, True, False):
         CM.record_tasks(s, on)
+        if on:
+            with pytest.raises(G.PastixGpuError):     # (the factor at hand was not recorded)
+                CM.task_records(s)
         s.numfact(A.values)
         if on:
             info, ns = CM.task_records(s)
