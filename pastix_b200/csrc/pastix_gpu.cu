@@ -1183,6 +1183,18 @@ static int make_fact_plan(pastix_gpu_t &C, int fmode, bool fp32, bool zc, PlanRo
     // TMA operands (3xTF32, persistent kernel): hi/lo mirrors, tensor maps of
     // the source cblks, split jobs of their off-diagonal rows per level
     C.tma = tma_mode;
+    if (C.tma) {
+        // the epilogue warps' larger share of registers comes out of what the launch got: compiled to fewer, they
+        // would wait for it for good
+        cudaFuncAttributes fa, fb;
+        PGPU_CHECK(cudaFuncGetAttributes(&fa, k_gemm_scatter_tc_tma<true, true>));
+        PGPU_CHECK(cudaFuncGetAttributes(&fb, k_gemm_scatter_tc_tma<true>));
+        if (std::min(fa.numRegs, fb.numRegs) < TMA_REGS_LAUNCH) {
+            fprintf(stderr, "pastix_gpu: the TMA kernel was compiled to %d registers, its split needs %d\n",
+                    std::min(fa.numRegs, fb.numRegs), TMA_REGS_LAUNCH);
+            return PASTIX_GPU_ERR_INTERNAL;
+        }
+    }
     C.split_ptr.assign(C.nlevels + 1, 0);
     C.h16 = C.tma && mixed_gemm_mode(C) == MG_3XF16;
     std::vector<int> mapidx_h;        // operand maps of each source cblk (TMA modes), for the tile descriptors

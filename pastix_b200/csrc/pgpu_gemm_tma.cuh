@@ -46,7 +46,8 @@ namespace pgpu {
 constexpr int TMA_THREADS = 384, TMA_EPI_WARPS = 8;
 constexpr int TMA_PROD_WARP = 8, TMA_MMA_WARP = 9;
 constexpr int TMA_REGS_EPI = 208, TMA_REGS_REST = 88;
-static_assert(2 * TMA_REGS_EPI + TMA_REGS_REST == 3 * 168, "register split");
+constexpr int TMA_REGS_LAUNCH = 168;
+static_assert(2 * TMA_REGS_EPI + TMA_REGS_REST == 3 * TMA_REGS_LAUNCH, "register split");
 constexpr int TMA_EPI_BYTES = TMA_EPI_WARPS * 32 * 32 * 4;   // a swizzled 32 x 32 float buffer per warp
 // operand maps per cblk: L panel, U panel (LU; LDL: the L rows times D), first / second diagonal-block
 // inverse, and in complex arithmetic the L / U panels as B operands (two real rows per row, see below)
